@@ -17,6 +17,7 @@
 #include "dsf_device.cuh"
 #include "dsf_math.cuh"
 #include "dsf_launch_v3.cuh"
+#include "dsf_pk_launch.cuh"
 
 #include <algorithm>
 #include <array>
@@ -80,6 +81,7 @@ struct dsf_engine {
     int n_sm = 0;
     size_t max_smem = 0;
     double *d_rotfit = nullptr;  // rotation-block fit (pinv blocks + sample directions) on this device
+    double *d_math = nullptr;    // tables of the FP64 exponential and sine (kMathTab doubles)
     // batched launches alternate between the call's stream and this one (under the batch launch lock)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -212,6 +214,7 @@ struct dsf_structure {
     // vector; sym_sign: that map's signs relative to the coset's first operation
     int electron = 0;            // HC: Mott-Bethe electron scattering
     int coset_size = 0;
+    PkForm pk;          // the operations' form for pk_kernel (cs = 0: none)
     int inv_pairs = 0;  // generic models: operations n/2 .. n-1 are the images of 0 .. n/2-1 under -1 at the origin
     int debug_stall = 0;  // dsf_debug_stall_next_call: the next call's kernel waits run out (timeout test)
     int tune_bps = 0, tune_ht = 0, tune_occ3 = 0;  // the autotuner's candidate for the next calls (bps 0: none)
@@ -238,10 +241,11 @@ struct dsf_structure {
         d_types_f, d_tcoeff, d_texp, d_tpow, d_texp_f, d_tpre_f, d_hkl, d_h2, d_h2f, d_hmult, d_cinv, d_table_f, d_table_d, d_perm, d_multw, d_dmat,
         d_raw, d_dtdf, d_gw_d, d_gw_f, d_facc, d_gacc, d_out, d_plm_lmax,
         d_rs_f, d_rs_d, d_tr_f, d_tr_d, d_trm_f, d_trm_d, d_err, d_hperm, d_cont, d_tile_lmax,
-        d_lcs, d_type_plm, d_type_lmax, d_atom_type0, d_step_f, d_step_d;
+        d_lcs, d_type_plm, d_type_lmax, d_atom_type0, d_step_f, d_step_d, d_pk_d;
     std::vector<int> hperm;  // line-ordered reflection -> caller's index
     int n_hkl_pad = 0;
     // resident tables per precision (0: FP32, 1: FP64), built when a call first needs them
+    bool pk_ok = false;  // the FP64 records of pk_kernel
     bool rs_ok[2] = {false, false}, tr_ok[2] = {false, false}, trm_ok[2] = {false, false};
     int n_tiles_plain = 0;   // tiles [0, n_tiles_plain) hold atoms without anisotropic ADPs
     int max_types_plain = 1, max_types_aniso = 1;
@@ -720,6 +724,66 @@ bool fractional_signs(dsf_structure *s, int cs)
     return true;
 }
 
+// The operations' form for pk_kernel: cosets of four or two consecutive operations whose relative maps flip axes as
+// a compiled sign group does (HC: the Cartesian maps of the harmonics too), the second half of the operations as
+// inversion images (generic models), or no cosets (cs = 1)
+PkForm pk_form_of(const dsf_structure *s)
+{
+    const int n = s->n_sym;
+    const bool hc = s->model == MODEL_HC;
+    // axes (bit mask) that operation op flips relative to operation ref on the fractional h'; -1: not such a map
+    auto mask = [&](int op, int ref) {
+        int m = 0;
+        const int *R = &s->sym_rot[9 * op], *Rr = &s->sym_rot[9 * ref];
+        for (int i = 0; i < 3; i++) {
+            bool same = true, flip = true;
+            for (int j = 0; j < 3; j++) {
+                same = same && R[3 * j + i] == Rr[3 * j + i];
+                flip = flip && R[3 * j + i] == -Rr[3 * j + i];
+            }
+            if (same == flip) return -1;  // neither, or a zero column
+            if (flip) m |= 1 << i;
+        }
+        if (hc)  // the harmonics' signs: the Cartesian map of the same coset
+            for (int i = 0; i < 3; i++)
+                if ((s->sym_sign[3 * op + i] < 0) != (((m >> i) & 1) != 0)) return -1;
+        return m;
+    };
+    auto cosets = [&](int cs, int a, int b) {
+        if (n % cs || (hc && s->coset_size != cs)) return false;
+        for (int op = 0; op < n; op++) {
+            const int j = op % cs;
+            if (mask(op, op - j) != (((j & 1) ? a : 0) ^ ((j & 2) ? b : 0))) return false;
+        }
+        return true;
+    };
+    PkForm f;
+    f.n_sym = n;
+    f.inv = !hc && s->inv_pairs != 0;
+    for (const int pat : {kPatD2, kPatC2hB})
+        if (cosets(4, pat & 7, pat >> 3)) {
+            f.cs = 4;
+            f.pat = pat;
+            return f;
+        }
+    for (const int a : {kPat2Y, kPat2Z, kPatInv})
+        if (cosets(2, a, 0)) {
+            f.cs = 2;
+            f.pat = a;
+            return f;
+        }
+    f.cs = 1;
+    f.inv = false;
+    return f;
+}
+
+// forms with compiled kernels: plain FP64
+bool pk_form_compiled(const dsf_structure *s, bool fp64)
+{
+    if (!fp64) return false;
+    return s->model == MODEL_HC ? pk_hc_form(s->pk, [](auto) {}) : pk_generic_form(s->pk, [](auto) {});
+}
+
 int sym_from_desc(dsf_engine *e, dsf_structure *s, const dsf_symmetry *sym)
 {
     if (!sym || sym->n_symops < 1 || sym->n_symops > kMaxSym)
@@ -755,6 +819,7 @@ int sym_from_desc(dsf_engine *e, dsf_structure *s, const dsf_symmetry *sym)
         }
         s->inv_pairs = pairs ? 1 : 0;
     }
+    s->pk = pk_form_of(s);
     s->centro_mode = 0;
     if (sym->centrosymmetric) {
         bool origin = true;
@@ -1040,8 +1105,15 @@ int ensure_tables(dsf_structure *s, bool fp64, bool mp)
     const int p = fp64 ? 1 : 0;
     const size_t esz = fp64 ? sizeof(double) : sizeof(float);
     const size_t row = 8 * (size_t)s->n_hkl_pad * std::max(1, s->n_types);
-    const bool built = !s->rs_ok[p] || !s->tr_ok[p] || (mp && !s->trm_ok[p]);
-    if (!s->rs_ok[p]) {
+    const bool pk = pk_form_compiled(s, fp64);
+    const bool built = (pk ? !s->pk_ok : !s->rs_ok[p]) || !s->tr_ok[p] || (mp && !s->trm_ok[p]);
+    if (pk && !s->pk_ok) {
+        const size_t rec = pk_rec_bytes<double>(s->model == MODEL_HC, s->n_sym, s->n_sym / s->pk.cs);
+        DSF_CUDA(s->d_pk_d.alloc(rec * (size_t)s->n_hkl_pad));
+        DSF_CUDA(launch_pk_prep(s->dev, s->n_hkl_pad, s->pk.cs, 2, s->d_pk_d.p, e->setup));
+        s->pk_ok = true;
+    }
+    if (!pk && !s->rs_ok[p]) {
         DevBuf &rs = fp64 ? s->d_rs_d : s->d_rs_f;
         DSF_CUDA(rs.alloc(rs_record_bytes(fp64) * (size_t)s->n_hkl_pad * s->n_sym));
         DSF_CUDA(launch_rs_prep(s->dev, s->n_hkl_pad, fp64 ? nullptr : rs.p, fp64 ? rs.p : nullptr, e->setup));
@@ -1320,6 +1392,25 @@ int dsf_engine_create(int device, dsf_engine **out)
         delete e;
         return DSF_ERR_CUDA;
     }
+    // tables of the FP64 kernels' exponential and sine, rounded from extended precision
+    std::vector<double> math(kMathTab);
+    const long double two_pi = 6.283185307179586476925286766559L;
+    for (int j = 0; j < kExpN; j++) math[j] = (double)std::exp2((long double)j / kExpN);
+    for (int j = 0; j < kSinLen; j++) {
+        const int q = j % kSinN, k = q * 4 / kSinN, r = q - k * (kSinN / 4);  // quadrant, rest: exact at quarter turns
+        const long double x = two_pi * r / kSinN;
+        const long double v = (k & 1) ? std::cos(x) : std::sin(x);
+        math[kExpN + j] = (double)((k & 2) ? -v : v);
+    }
+    ce = cudaMalloc(&e->d_math, sizeof(double) * kMathTab);
+    if (ce == cudaSuccess) ce = cudaMemcpy(e->d_math, math.data(), sizeof(double) * kMathTab, cudaMemcpyHostToDevice);
+    if (ce != cudaSuccess) {
+        cudaStreamDestroy(e->stream);
+        cudaStreamDestroy(e->setup);
+        if (e->d_math) cudaFree(e->d_math);
+        delete e;
+        return DSF_ERR_CUDA;
+    }
     cudaDeviceGetAttribute(&e->n_sm, cudaDevAttrMultiProcessorCount, device);
     int smem = 0;
     cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -1339,6 +1430,7 @@ int dsf_engine_destroy(dsf_engine *e)
     if (e->ev_fork) cudaEventDestroy(e->ev_fork);
     if (e->ev_join) cudaEventDestroy(e->ev_join);
     if (e->d_rotfit) cudaFree(e->d_rotfit);
+    if (e->d_math) cudaFree(e->d_math);
     delete e;
     return DSF_OK;
 }
@@ -1675,7 +1767,7 @@ int dsf_structure_destroy(dsf_structure *s)
                       &s->d_dtdf, &s->d_gw_d, &s->d_gw_f, &s->d_facc, &s->d_gacc, &s->d_out, &s->d_plm_lmax,
                       &s->d_rs_f, &s->d_rs_d, &s->d_tr_f, &s->d_tr_d, &s->d_trm_f, &s->d_trm_d, &s->d_err,
                       &s->d_hperm, &s->d_cont, &s->d_tile_lmax, &s->d_lcs, &s->d_type_plm, &s->d_type_lmax,
-                      &s->d_atom_type0, &s->d_step_f, &s->d_step_d};
+                      &s->d_atom_type0, &s->d_step_f, &s->d_step_d, &s->d_pk_d};
     for (DevBuf *b : bufs) b->release();
     if (s->ev_begin) cudaEventDestroy(s->ev_begin);
     if (s->ev_end) cudaEventDestroy(s->ev_end);
@@ -1700,6 +1792,7 @@ int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl)
         s->n_hkl_pad = 0;
         s->have_hkl = true;
         for (int p = 0; p < 2; p++) s->rs_ok[p] = s->tr_ok[p] = s->trm_ok[p] = false;
+        s->pk_ok = false;
         refresh_dev(s);
         return DSF_OK;
     }
@@ -1777,6 +1870,7 @@ int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl)
     refresh_dev(s);
     // resident per-(reflection, operation) and radial tables: FP32 now, FP64 on the first FP64 call
     for (int p = 0; p < 2; p++) s->rs_ok[p] = s->tr_ok[p] = s->trm_ok[p] = false;
+    s->pk_ok = false;
     int rc2 = ensure_tables(s, false, false);
     if (rc2) return rc2;
     DSF_CUDA(cudaStreamSynchronize(e->setup));
@@ -1895,7 +1989,7 @@ int64_t dsf_structure_device_bytes(const dsf_structure *s)
                             &s->d_dmat, &s->d_raw, &s->d_dtdf, &s->d_gw_d, &s->d_gw_f, &s->d_facc, &s->d_gacc,
                             &s->d_out, &s->d_plm_lmax, &s->d_rs_f, &s->d_rs_d, &s->d_tr_f, &s->d_tr_d,
                             &s->d_trm_f, &s->d_trm_d, &s->d_err, &s->d_hperm, &s->d_cont, &s->d_tile_lmax,
-                            &s->d_lcs, &s->d_type_plm, &s->d_type_lmax, &s->d_atom_type0, &s->d_step_f, &s->d_step_d};
+                            &s->d_lcs, &s->d_type_plm, &s->d_type_lmax, &s->d_atom_type0, &s->d_step_f, &s->d_step_d, &s->d_pk_d};
     int64_t b = 0;
     for (const DevBuf *p : bufs) b += (int64_t)p->bytes;
     return b;
@@ -2101,6 +2195,67 @@ static bool inv_kernel(const dsf_structure *s, bool fp64)
     return s->inv_pairs && !fp64 && s->model != MODEL_HC && table_count_compiled(s->n_sym);
 }
 
+// one structure's launch of pk_kernel: every tile, reflection chunks that give about `bps` blocks per SM, at least
+// one sub-tile each.  Sub-tiles of 16 reflections where the shared-memory budget allows (two blocks per SM); shorter
+// ones only where the reflections are too few to give every SM its blocks.
+static int launch_pk_structure(dsf_structure *s, bool fp64, bool mp, bool grad, int bps, int ht_cap, cudaStream_t st)
+{
+    dsf_engine *e = s->eng;
+    CallBuffers C;
+    C.gw_d = s->d_gw_d.as<double2>();
+    C.gw_f = s->d_gw_f.as<float2>();
+    C.f_acc = s->d_facc.as<double2>();
+    C.g_acc = s->d_gacc.as<double>();
+    PkLaunch L{};
+    L.max_types = std::max(s->n_tiles_plain > 0 ? s->max_types_plain : 1,
+                           s->n_tiles_plain < s->n_tiles ? s->max_types_aniso : 1);
+    L.n_hkl_pad = s->n_hkl_pad;
+    L.n_plain = s->n_tiles_plain;
+    L.pk = s->d_pk_d.p;
+    L.tr = fp64 ? s->d_tr_d.p : s->d_tr_f.p;
+    L.trm = fp64 ? s->d_trm_d.p : s->d_trm_f.p;
+    L.cont = s->d_cont.as<int>();
+    L.tile_lmax = s->d_tile_lmax.as<int>();
+    L.math = e->d_math;
+    L.error = s->d_err.as<int>();
+    L.stall_first = s->debug_stall;
+    s->debug_stall = 0;
+    const bool mp_hc = mp && s->model == MODEL_HC, gr = grad || mp_hc || s->model != MODEL_HC;
+    const int ncos = s->n_sym / s->pk.cs;
+    auto bytes = [&](int ht) {
+        return mp_hc ? pk_smem_bytes<double, true>(s->model, ht, s->n_sym, ncos, L.max_types, true)
+                     : pk_smem_bytes<double, false>(s->model, ht, s->n_sym, ncos, L.max_types, gr);
+    };
+    const int n_chunks0 = chunk_count(e, s->n_tiles, s->n_hkl, bps);
+    const int want = std::max(1, (s->n_hkl + n_chunks0 - 1) / n_chunks0);
+    // two blocks per SM with sub-tiles of 16 or 8 reflections, else one block with the longest that fits
+    int ht = kMaxHT;
+    if (bytes(8) > 110 * 1024)
+        while (ht > 4 && bytes(ht) > e->max_smem) ht /= 2;
+    else if (bytes(ht) > 110 * 1024)
+        ht = 8;
+    while (ht > 4 && want < ht) ht /= 2;
+    while (ht_cap >= 4 && ht > ht_cap) ht /= 2;
+    if (bytes(ht) > e->max_smem) return fail(e, DSF_ERR_UNSUPPORTED, "shared-memory tile does not fit this device");
+    L.ht = ht;
+    L.hkl_chunk = (want + ht - 1) / ht * ht;
+    PkArgs A;
+    A.S = &s->dev;
+    A.C = &C;
+    A.L = &L;
+    A.form = s->pk;
+    A.n_tiles = s->n_tiles;
+    A.n_chunks = (s->n_hkl + L.hkl_chunk - 1) / L.hkl_chunk;
+    A.smem = bytes(ht);
+    A.st = st;
+    if (s->model == MODEL_IAM) DSF_CUDA(launch_pk_f64_iam(A));
+    else if (s->model == MODEL_TABLE) DSF_CUDA(launch_pk_f64_table(A));
+    else if (mp_hc) DSF_CUDA(launch_pk_f64_hc_mp(A));
+    else if (grad) DSF_CUDA(launch_pk_f64_hc(A));
+    else DSF_CUDA(launch_pk_f64_hc_f(A));
+    return DSF_OK;
+}
+
 // a call on an empty reflection set: no F, the requested derivatives zero (the reference's engines sum over no
 // reflections); no kernels
 static int empty_call(dsf_structure *s, int flags, const dsf_outputs *out, cudaStream_t st)
@@ -2136,7 +2291,8 @@ int dsf_calculate_device(dsf_structure *s, int precision, int flags, const doubl
     CallBuffers C;
     SfLaunch L;
     SignTable G;
-    call_buffers(s, fp64, C, L, G);
+    const bool pk = pk_form_compiled(s, fp64);
+    if (!pk) call_buffers(s, fp64, C, L, G);
     if (!s->ev_begin) {
         DSF_CUDA(cudaEventCreate(&s->ev_begin));
         DSF_CUDA(cudaEventCreate(&s->ev_end));
@@ -2145,9 +2301,13 @@ int dsf_calculate_device(dsf_structure *s, int precision, int flags, const doubl
     int bps, ht_cap, occ3;
     call_shape(s, fp64, mp, grad, bps, ht_cap, occ3);
     DSF_CUDA(cudaEventRecord(s->ev_begin, st));
+    if (pk) {
+        if ((rc = launch_pk_structure(s, fp64, mp, grad, bps, ht_cap, st))) return rc;
+        launches++;
+    }
     // one launch per ADP kind (tiles [0, n_tiles_plain) without anisotropic ADPs), reflection chunks of
     // chunk_count
-    for (int kind = 0; kind < 2; kind++) {
+    for (int kind = 0; kind < 2 && !pk; kind++) {
         int nt, n_chunks;
         size_t smem;
         const int ntk = kind ? s->n_tiles - s->n_tiles_plain : s->n_tiles_plain;
@@ -2421,6 +2581,12 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
     for (int i = 0; i < n; i++) {
         dsf_structure *s = structures[i];
         const bool mp = (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC;
+        if (pk_form_compiled(s, fp64)) {
+            const bool grad = (flags & (DSF_D_XYZ | DSF_D_ADP | DSF_D_OCC | DSF_D_MULTIPOLE)) != 0;
+            if ((rc = launch_pk_structure(s, fp64, mp, grad, 75, 0, st))) return rc;
+            launches++;
+            continue;
+        }
         CallBuffers C;
         SfLaunch L;
         SignTable G;

@@ -1,0 +1,95 @@
+// Launch helpers of pk_kernel: one instantiation per (value type, model, derivatives, operation count, coset size,
+// sign group); the translation units dsf_pk_*.cu hold the instantiations.
+#pragma once
+#include "dsf_pk_kernel.cuh"
+
+namespace dsf {
+
+// the symmetry form of a launch: n_sym operations in cosets of cs that form the sign group pat (cs = 4: kPatD2,
+// kPatC2hB; cs = 2: the mask of the axes that the second operation flips); inv: the second half of the operations
+// are the images of the first half under an inversion at the origin
+struct PkForm {
+    int n_sym = 0, cs = 0, pat = 0;
+    bool inv = false;
+};
+
+struct PkArgs {
+    const DevStructure *S = nullptr;
+    const CallBuffers *C = nullptr;
+    const PkLaunch *L = nullptr;
+    PkForm form;
+    int n_tiles = 0, n_chunks = 0;
+    size_t smem = 0;
+    cudaStream_t st = nullptr;
+};
+
+constexpr int kPat2Y = 5, kPat2Z = 3, kPatInv = 7;  // cs = 2: a two-fold axis along b, along c, an inversion
+
+// runs f with the compile-time form that equals `f0`, one of the compiled ones of the model; false when none does.
+//   HC (operations without the inversion): P1 and P-1; P2_1, P2_1/c, C2/c; P4_1; 222; 422
+//   other models (all operations modulo centring): 1; 2; -1; 222; 2/m; mmm; any eight
+template <int N_, int CS_, int PAT_, bool INV_ = false>
+struct PkC {
+    static constexpr int N = N_, CS = CS_, PAT = PAT_;
+    static constexpr bool INV = INV_;
+};
+template <typename C>
+inline bool pk_is(const PkForm &f)
+{
+    return f.n_sym == C::N && f.cs == C::CS && (C::CS == 1 || f.pat == C::PAT) && f.inv == C::INV;
+}
+template <typename F>
+inline bool pk_hc_form(const PkForm &f, F &&go)
+{
+    if (pk_is<PkC<1, 1, 0> >(f)) return go(PkC<1, 1, 0>{}), true;
+    if (pk_is<PkC<2, 2, kPat2Y> >(f)) return go(PkC<2, 2, kPat2Y>{}), true;
+    if (pk_is<PkC<4, 2, kPat2Z> >(f)) return go(PkC<4, 2, kPat2Z>{}), true;
+    if (pk_is<PkC<4, 4, kPatD2> >(f)) return go(PkC<4, 4, kPatD2>{}), true;
+    if (pk_is<PkC<8, 4, kPatD2> >(f)) return go(PkC<8, 4, kPatD2>{}), true;
+    return false;
+}
+template <typename F>
+inline bool pk_generic_form(const PkForm &f, F &&go)
+{
+    if (pk_is<PkC<1, 1, 0> >(f)) return go(PkC<1, 1, 0>{}), true;
+    if (pk_is<PkC<2, 2, kPat2Y> >(f)) return go(PkC<2, 2, kPat2Y>{}), true;
+    if (pk_is<PkC<2, 2, kPatInv, true> >(f)) return go(PkC<2, 2, kPatInv, true>{}), true;
+    if (pk_is<PkC<4, 4, kPatD2> >(f)) return go(PkC<4, 4, kPatD2>{}), true;
+    if (pk_is<PkC<4, 4, kPatC2hB, true> >(f)) return go(PkC<4, 4, kPatC2hB, true>{}), true;
+    if (pk_is<PkC<8, 4, kPatD2, true> >(f)) return go(PkC<8, 4, kPatD2, true>{}), true;
+    if (pk_is<PkC<8, 1, 0> >(f)) return go(PkC<8, 1, 0>{}), true;
+    return false;
+}
+
+template <typename V, int MODEL, bool MP, bool GRAD, typename C>
+cudaError_t launch_pk(const PkArgs &A)
+{
+    auto k = pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A.smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(A.n_tiles, A.n_chunks), pk_threads<V>(), A.smem, A.st>>>(*A.S, *A.C, *A.L);
+    return cudaGetLastError();
+}
+
+// a form's launch, cudaErrorInvalidValue where the form is not compiled (the engine asks pk_form_compiled first)
+template <typename V, int MODEL, bool MP, bool GRAD>
+cudaError_t dispatch_pk(const PkArgs &A)
+{
+    cudaError_t e = cudaErrorInvalidValue;
+    auto go = [&](auto c) { e = launch_pk<V, MODEL, MP, GRAD, decltype(c)>(A); };
+    if constexpr (MODEL == MODEL_HC) pk_hc_form(A.form, go);
+    else pk_generic_form(A.form, go);
+    return e;
+}
+
+// per-translation-unit entries
+cudaError_t launch_pk_f64_hc(const PkArgs &A);
+cudaError_t launch_pk_f64_hc_mp(const PkArgs &A);
+cudaError_t launch_pk_f64_hc_f(const PkArgs &A);
+cudaError_t launch_pk_f64_iam(const PkArgs &A);
+cudaError_t launch_pk_f64_table(const PkArgs &A);
+
+// record tables (dsf_prep_kernels.cu): kind 0: F2 slots (duplicated floats), 1: float slots, 2: double slots
+cudaError_t launch_pk_prep(const DevStructure &S, int n_hkl_pad, int cs, int kind, void *out, cudaStream_t st);
+
+}  // namespace dsf

@@ -15,7 +15,7 @@
 // Rows past the last reflection (padding to a multiple of 16) are zero.
 #include "dsf_device.cuh"
 #include "dsf_math.cuh"
-#include "dsf_sf_kernel.cuh"
+#include "dsf_pk_launch.cuh"
 
 namespace dsf {
 
@@ -193,6 +193,72 @@ cudaError_t launch_tr_prep(const DevStructure &S, int n_hkl_pad, void *tr_f, voi
     double *td = mp ? nullptr : (double *)tr_d, *md = mp ? (double *)trm_d : nullptr;
     if (tf || mf) tr_prep_kernel<float><<<grid, 128, 0, st>>>(S, n_hkl_pad, tf, mf, mp);
     if (td || md) tr_prep_kernel<double><<<grid, 128, 0, st>>>(S, n_hkl_pad, td, md, mp);
+    return cudaGetLastError();
+}
+
+// Records of pk_kernel: per (reflection, operation) the integers of the exact phase, per (reflection, coset) the
+// harmonics (HC), h' and its monomials of the coset's first operation, in slots of V; rows past n_hkl are zero.
+template <typename V>
+__global__ void pk_prep_kernel(DevStructure S, int n_hkl_pad, int cs, unsigned char *out)
+{
+    using R = typename VTraits<V>::R;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nS = S.n_sym;
+    if (i >= n_hkl_pad * nS) return;
+    const int h = i / nS, s = i - h * nS;
+    const bool hc = S.model == MODEL_HC;
+    unsigned char *rec = out + pk_rec_bytes<V>(hc, nS, nS / cs) * (size_t)h;
+    PkOp op;
+    int hp[3] = {0, 0, 0}, tr = 0;
+    if (h < S.n_hkl) {
+        const int4 hv = S.hkl[h];
+        const int *Rm = S.sym_rot + 9 * s, *t = S.sym_t24 + 3 * s;
+        for (int j = 0; j < 3; j++) hp[j] = hv.x * Rm[j] + hv.y * Rm[3 + j] + hv.z * Rm[6 + j];
+        tr = (hv.x * t[0] + hv.y * t[1] + hv.z * t[2]) % 24;
+        if (tr < 0) tr += 24;
+    }
+    for (int j = 0; j < 3; j++) op.h[j] = hp[j];
+    if constexpr (sizeof(R) == 4) {
+        op.h[3] = (int)(uint32_t)((((uint64_t)tr << 32) + 12u) / 24u);
+        for (int j = 0; j < 3; j++) op.hf[j] = (float)hp[j];
+        op.hf[3] = 0.f;
+    } else {
+        op.h[3] = 0;
+        op.tq = (uint64_t)tr * 0x0aaaaaaaaaaaaaaaull + (uint64_t)(tr * 16 + 12) / 24u;  // tr 2^64 / 24
+        op.hf[2] = op.hf[3] = 0.f;
+    }
+    reinterpret_cast<PkOp *>(rec)[s] = op;
+    if (s % cs != 0) return;
+    V *dst = reinterpret_cast<V *>(rec + sizeof(PkOp) * nS) + pk_slots<V>(hc) * (s / cs);
+    R v[36];
+    for (int q = 0; q < 36; q++) v[q] = R(0);
+    const int off = hc ? 25 : 0;
+    if (hc && h < S.n_hkl) {
+        const double cx = S.B[0] * hp[0] + S.B[1] * hp[1] + S.B[2] * hp[2];
+        const double cy = S.B[3] * hp[0] + S.B[4] * hp[1] + S.B[5] * hp[2];
+        const double cz = S.B[6] * hp[0] + S.B[7] * hp[1] + S.B[8] * hp[2];
+        const double n2 = cx * cx + cy * cy + cz * cz;
+        if (n2 > 1e-20) {  // F(000): no deformation term
+            const double inv = 1.0 / sqrt(n2);
+            double y[25];
+            harmonic_polys<double>(cx * inv, cy * inv, cz * inv, y);
+            for (int q = 0; q < 25; q++) v[q] = R(y[q] * kDensityNorm[q]);
+        }
+    }
+    const R a = R(hp[0]), b = R(hp[1]), c = R(hp[2]);
+    v[off] = a; v[off + 1] = b; v[off + 2] = c;
+    v[off + 3] = a * a; v[off + 4] = b * b; v[off + 5] = c * c;
+    v[off + 6] = R(2) * a * b; v[off + 7] = R(2) * a * c; v[off + 8] = R(2) * b * c;
+    for (int q = 0; q < pk_slots<V>(hc); q++) dst[q] = vdup<V>(v[q]);
+}
+
+cudaError_t launch_pk_prep(const DevStructure &S, int n_hkl_pad, int cs, int kind, void *out, cudaStream_t st)
+{
+    const int n = n_hkl_pad * S.n_sym;
+    unsigned char *o = static_cast<unsigned char *>(out);
+    if (kind == 0) pk_prep_kernel<F2><<<(n + 127) / 128, 128, 0, st>>>(S, n_hkl_pad, cs, o);
+    else if (kind == 1) pk_prep_kernel<float><<<(n + 127) / 128, 128, 0, st>>>(S, n_hkl_pad, cs, o);
+    else pk_prep_kernel<double><<<(n + 127) / 128, 128, 0, st>>>(S, n_hkl_pad, cs, o);
     return cudaGetLastError();
 }
 

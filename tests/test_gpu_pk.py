@@ -1,0 +1,85 @@
+"""pk_kernel (dsf_pk_kernel.cuh) against the CPU oracle where its tiling can go wrong: tiles of one atom, around the
+32-, 64- and 128-atom marks (a small tile's warps share out the reflections), more than 32 types, reflection counts
+around the sub-tile length, excluded atoms, every compiled symmetry form.
+
+Tolerances: the plain form is held to the parity bar of the FP64 path (1e-10 relative), a factor 1e4 above the
+rounding of these sums."""
+import numpy as np
+import pytest
+
+from conftest import rel_f, rel_norm
+from discamb_gb300 import api, workloads as W
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+KEYS = ("d_xyz", "d_adp", "d_occ")
+
+
+def cut(st, n_hkl):
+    idx = np.linspace(0, st.n_hkl - 1, n_hkl + 2).astype(int)[1:-1]  # not the first: an extinct axial one
+    st.hkl, st.dtdf = np.ascontiguousarray(st.hkl[idx]), st.dtdf[idx]
+    return st
+
+
+def check(got, ref, tol, keys=KEYS):
+    assert rel_f(got["f"], ref["f"]) < tol
+    largest = max(np.linalg.norm(np.ravel(ref[k])) for k in keys)
+    for k in keys:
+        if np.linalg.norm(np.ravel(ref[k])) > 1e-12 * largest:
+            assert rel_norm(got[k], ref[k]) < tol, k
+        else:  # a class that symmetry makes zero (one extinct reflection): rounding on both sides
+            assert np.linalg.norm(np.ravel(got[k])) < 1e-12 * largest, k
+
+
+def padded(ref, st):
+    out = np.zeros((st.n_atoms, 6))
+    for i, a in enumerate(ref["d_adp"]):
+        out[i, :len(a)] = a
+    return dict(ref, d_adp=out)
+
+
+@pytest.mark.parametrize("n_atoms,n_hkl", [(1, 1), (2, 3), (31, 17), (33, 16), (65, 15), (70, 33), (129, 5), (200, 40)])
+@pytest.mark.parametrize("sg", ["P1", "P21/c", "P212121", "P41"])
+def test_fp64_tile_edges(engine, sg, n_atoms, n_hkl):
+    st = cut(W.small_case(sg, n_atoms=n_atoms, stol_max=0.45, seed=900 + n_atoms), n_hkl)
+    ref = padded(O.compute(st, multipoles=True), st)
+    calc = api.HcCalculator(engine, st)
+    keys = KEYS + ("d_pval", "d_plm", "d_kappa", "d_kappa_p")
+    check(calc.calculate(st.dtdf, multipoles=True, adp_layout="padded"), ref, 1e-10, keys)
+    check(calc.calculate(st.dtdf, adp_layout="padded"), ref, 1e-10)
+    assert rel_f(calc.calculate(st.dtdf, derivatives=())["f"], ref["f"]) < 1e-10
+
+
+@pytest.mark.parametrize("sg", ["P1", "P-1", "P21", "P21/c", "C2/c", "P212121", "Pbca", "P43212", "P3"])
+def test_fp64_excluded_atoms_every_form(engine, sg):
+    st = W.small_case(sg, n_atoms=37, stol_max=0.35, seed=77)
+    include = np.ones(37, dtype=np.int32)
+    include[::3] = 0
+    st.include = include.astype(bool)
+    rng = np.random.default_rng(3)
+    nt = int(st.atom_type.max()) + 1
+    iam = dict(ngauss=np.full(nt, 4, np.int32), a=rng.uniform(.5, 3, (nt, 5)), b=rng.uniform(.5, 30, (nt, 5)),
+               c=rng.uniform(0, .5, nt))
+    rots = api.all_ops_mod_centering(st.sg)[0]
+    n_ops = len(rots)
+    # the oracle sums the centred copies of every operation too: the same form factors for the same rotation
+    every = [next(k for k in range(n_ops) if np.array_equal(rots[k], r)) for r in st.sg.rot]
+    table = rng.normal(size=(st.n_hkl, n_ops, 37)) + 1j * rng.normal(size=(st.n_hkl, n_ops, 37))
+    # values the widening of complex64 tables treats apart: zero, subnormal
+    table[0, 0, 1], table[0, 0, 2] = 0.0, 1e-41
+    for calc, ref in ((api.HcCalculator(engine, st), O.compute(st)),
+                      (api.IamCalculator(engine, st, iam), O.compute(st, model="iam", iam=iam)),
+                      (api.TabulatedCalculator(engine, st, table), O.compute(st, model="table", table=table[:, every])),
+                      (api.TabulatedCalculator(engine, st, table, fp32_table=True),
+                       O.compute(st, model="table", table=table[:, every].astype(np.complex64).astype(np.complex128)))):
+        got = calc.calculate(st.dtdf, include=include, adp_layout="padded")
+        check(got, padded(ref, st), 1e-10)
+
+
+def test_fp64_temperature_factors_far_out(engine):
+    """Displacements whose temperature factors underflow (zero there) or grow (not positive definite)."""
+    st = W.small_case("P21/c", n_atoms=9, stol_max=0.5, seed=5)
+    for i in range(st.n_atoms):
+        a = np.array(st.adp[i])
+        st.adp[i] = list(a * (4000.0 if i % 3 == 0 else -0.5 if i % 3 == 1 else 1.0))
+    check(api.HcCalculator(engine, st).calculate(st.dtdf, adp_layout="padded"), padded(O.compute(st), st), 1e-10)
