@@ -549,8 +549,8 @@ class _Calculator:
         """dsf_autotune: times this structure's call over a few tile shapes and
         keeps the fastest for every later call of structures of the same shape
         key.  Returns dict(blocks_per_sm, ht, occupancy, ms) of the chosen
-        shape (ht 0: the longest shared-memory sub-tile; occupancy 3: the
-        register-capped form, 0: the compiler's registers)."""
+        shape (ht 0: the longest shared-memory sub-tile; occupancy: always
+        0)."""
         bps, ht, occ, ms = C.c_int(0), C.c_int(0), C.c_int(0), C.c_double(0)
         self.engine.check(self.lib.dsf_autotune(self.h, int(precision), _flags(derivatives, multipoles), C.byref(bps),
                                                 C.byref(ht), C.byref(occ), C.byref(ms)), "autotune")

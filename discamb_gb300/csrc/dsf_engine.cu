@@ -87,7 +87,7 @@ struct dsf_engine {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // tile shapes chosen by the autotuner, per shape key (tune_key): blocks per SM the reflection chunks
     // aim at, and the sub-tile length (0: the longest the shared-memory budget allows)
-    std::map<std::string, std::array<int, 3> > tuned;  // blocks per SM, sub-tile cap, register-capped form
+    std::map<std::string, std::array<int, 3> > tuned;  // blocks per SM, sub-tile cap, 0
     std::mutex tune_mtx;
 };
 
@@ -194,6 +194,14 @@ void adp_param_map(const double *A, double *A6)
         }
 }
 
+// the tiles of a structure for pk_kernel (PkTiles)
+struct PkMap {
+    std::vector<int> slot;   // [n_tiles][kTileAtoms] sorted atom, -1: empty
+    std::vector<int4> info;
+    int n_tiles = 0, n_plain = 0, max_types = 1, used = 0;  // used: slots in use, holes of the pairs included
+    DevBuf d_slot, d_ltype, d_info, d_types;
+};
+
 }  // namespace
 
 struct dsf_structure {
@@ -214,10 +222,12 @@ struct dsf_structure {
     // vector; sym_sign: that map's signs relative to the coset's first operation
     int electron = 0;            // HC: Mott-Bethe electron scattering
     int coset_size = 0;
+    PkMap pkm[2];       // pk_kernel's tiles: pairs of one type (two atoms per thread, HC), dense
+    bool pk_pairs = false;  // the pairs leave few slots empty: FP32 HC calls take two atoms per thread
     PkForm pk;          // the operations' form for pk_kernel (cs = 0: none)
     int inv_pairs = 0;  // generic models: operations n/2 .. n-1 are the images of 0 .. n/2-1 under -1 at the origin
     int debug_stall = 0;  // dsf_debug_stall_next_call: the next call's kernel waits run out (timeout test)
-    int tune_bps = 0, tune_ht = 0, tune_occ3 = 0;  // the autotuner's candidate for the next calls (bps 0: none)
+    int tune_bps = 0, tune_ht = 0;  // the autotuner's candidate for the next calls (bps 0: none)
     int pending = 0;      // a dsf_submit call of this structure not yet completed by dsf_poll
     std::vector<int> sym_sign;   // [n_sym][3] Cartesian
     std::vector<int> sym_fsign;  // [n_sym][3] fractional h' components
@@ -241,11 +251,11 @@ struct dsf_structure {
         d_types_f, d_tcoeff, d_texp, d_tpow, d_texp_f, d_tpre_f, d_hkl, d_h2, d_h2f, d_hmult, d_cinv, d_table_f, d_table_d, d_perm, d_multw, d_dmat,
         d_raw, d_dtdf, d_gw_d, d_gw_f, d_facc, d_gacc, d_out, d_plm_lmax,
         d_rs_f, d_rs_d, d_tr_f, d_tr_d, d_trm_f, d_trm_d, d_err, d_hperm, d_cont, d_tile_lmax,
-        d_lcs, d_type_plm, d_type_lmax, d_atom_type0, d_step_f, d_step_d, d_pk_d;
+        d_lcs, d_type_plm, d_type_lmax, d_atom_type0, d_step_f, d_step_d, d_pk[3];
     std::vector<int> hperm;  // line-ordered reflection -> caller's index
     int n_hkl_pad = 0;
     // resident tables per precision (0: FP32, 1: FP64), built when a call first needs them
-    bool pk_ok = false;  // the FP64 records of pk_kernel
+    bool pk_ok[3] = {false, false, false};  // pk_kernel's records: two atoms per thread, one (FP32), FP64 (pk_kind)
     bool rs_ok[2] = {false, false}, tr_ok[2] = {false, false}, trm_ok[2] = {false, false};
     int n_tiles_plain = 0;   // tiles [0, n_tiles_plain) hold atoms without anisotropic ADPs
     int max_types_plain = 1, max_types_aniso = 1;
@@ -471,6 +481,7 @@ struct PrePostBatch {
     PrePostItem item[kPrePostItems];
 };
 static_assert(sizeof(PrePostBatch) <= 32000, "kernel parameters hold at most 32764 bytes");
+static_assert(sizeof(dsf::PkBatch) <= 32000, "kernel parameters hold at most 32764 bytes");
 static_assert(sizeof(dsf::SfBatch) <= 32000, "kernel parameters hold at most 32764 bytes");
 
 __global__ void batch_pre_kernel(const __grid_constant__ PrePostBatch B)
@@ -777,11 +788,16 @@ PkForm pk_form_of(const dsf_structure *s)
     return f;
 }
 
-// forms with compiled kernels: plain FP64
-bool pk_form_compiled(const dsf_structure *s, bool fp64)
+// the record kind (and thread value) pk_kernel takes a call in: 0 FP32 with two atoms per thread, 1 FP32 with one
+// (multipole adjoint; a type per atom), 2 FP64; -1: the call's form or model has no pk_kernel (FP32 tables stream through registers in
+// sf_grad_body; sign groups and operation counts that are not compiled)
+int pk_kind(const dsf_structure *s, bool fp64, bool mp)
 {
-    if (!fp64) return false;
-    return s->model == MODEL_HC ? pk_hc_form(s->pk, [](auto) {}) : pk_generic_form(s->pk, [](auto) {});
+    if (s->model == MODEL_TABLE && !fp64) return -1;
+    const bool form = s->model == MODEL_HC ? pk_hc_form(s->pk, [](auto) {}) : pk_generic_form(s->pk, [](auto) {});
+    if (!form) return -1;
+    if (fp64) return 2;
+    return s->model == MODEL_HC && (mp || !s->pk_pairs) ? 1 : 0;
 }
 
 int sym_from_desc(dsf_engine *e, dsf_structure *s, const dsf_symmetry *sym)
@@ -918,6 +934,33 @@ int upload(dsf_engine *e, DevBuf &b, const T *src, size_t n)
     return DSF_OK;
 }
 
+// highest l of the populations of a type that are not zero, and of all that it has
+int type_lmax(const dsf_structure *s, int t, bool used)
+{
+    if (s->model != MODEL_HC) return -1;
+    return used ? s->trad[t].lmax_used : std::min(std::min(s->type_nl[t] - 1, s->trad[t].n_def - 1), 4);
+}
+
+// the per-tile highest l of pk_kernel's tiles (they follow the populations)
+int upload_pk_info(dsf_structure *s)
+{
+    for (PkMap &m : s->pkm) {
+        for (int t = 0; t < m.n_tiles; t++) {
+            m.info[t].z = m.info[t].w = -1;
+            for (int i = 0; i < m.info[t].x; i++) {
+                const int a = m.slot[(size_t)t * kTileAtoms + i];
+                if (a < 0) continue;
+                const int ty = s->atom_type[s->perm[a]];
+                m.info[t].z = std::max(m.info[t].z, type_lmax(s, ty, true));
+                m.info[t].w = std::max(m.info[t].w, type_lmax(s, ty, false));
+            }
+        }
+        int rc = upload(s->eng, m.d_info, m.info.data(), m.info.size());
+        if (rc) return rc;
+    }
+    return DSF_OK;
+}
+
 int compute_global_plm(dsf_structure *s)
 {
     dsf_engine *e = s->eng;
@@ -959,7 +1002,7 @@ int compute_global_plm(dsf_structure *s)
             tl[t] = std::max(tl[t], s->trad[s->atom_type[s->perm[a]]].lmax_used);
     if ((rc = upload(e, s->d_tile_lmax, tl.data(), tl.size()))) return rc;
     if ((rc = upload(e, s->d_plm_lmax, lmx.data(), lmx.size()))) return rc;
-    return DSF_OK;
+    return upload_pk_info(s);
 }
 
 // pre_hkl_loop_sf_calc: l used in the sum and the deformation normalisation
@@ -1001,15 +1044,76 @@ int build_type_radial(dsf_structure *s, const dsf_hc_model *m)
     return DSF_OK;
 }
 
+// pk_kernel's tiles over the sorted atoms (PkTiles); host arrays and uploads
+int build_pk_map(dsf_structure *s, PkMap &m, bool by_type, bool pairs)
+{
+    const int n = s->n_atoms;
+    m = PkMap{};
+    std::vector<int> slots, ltype, types, d_ltype, d_types;
+    int kind = 0, high = 0, prev = -1;
+    auto close = [&]() {
+        if (slots.empty()) return;
+        if (pairs && slots.size() % 2) {
+            slots.push_back(-1);
+            ltype.push_back(0);
+        }
+        m.info.push_back(make_int4((int)slots.size(), (int)types.size(), -1, -1));
+        m.used += (int)slots.size();
+        m.max_types = std::max(m.max_types, (int)types.size());
+        if (!kind) m.n_plain++;
+        slots.resize(kTileAtoms, -1);
+        ltype.resize(kTileAtoms, 0);
+        types.resize(kMaxTileTypes, 0);
+        m.slot.insert(m.slot.end(), slots.begin(), slots.end());
+        d_ltype.insert(d_ltype.end(), ltype.begin(), ltype.end());
+        d_types.insert(d_types.end(), types.begin(), types.end());
+        m.n_tiles++;
+        slots.clear();
+        ltype.clear();
+        types.clear();
+    };
+    for (int a = 0; a < n; a++) {
+        const int o = s->perm[a], t = by_type ? s->atom_type[o] : 0;
+        const int k = s->adpk[o] == 6, h = type_lmax(s, s->atom_type[o], true) >= 3;
+        if (k != kind || h != high) close();
+        kind = k;
+        high = h;
+        if (pairs && t != prev && slots.size() % 2) {  // the type before ends inside a pair
+            slots.push_back(-1);
+            ltype.push_back(0);
+        }
+        prev = t;
+        if ((int)slots.size() == kTileAtoms) close();
+        size_t li = std::find(types.begin(), types.end(), t) - types.begin();
+        if (li == types.size()) {
+            if ((int)types.size() == kMaxTileTypes) {
+                close();
+                li = 0;
+            }
+            types.push_back(t);
+        }
+        slots.push_back(a);
+        ltype.push_back((int)li);
+    }
+    close();
+    int rc;
+    if ((rc = upload(s->eng, m.d_slot, m.slot.data(), m.slot.size()))) return rc;
+    if ((rc = upload(s->eng, m.d_ltype, d_ltype.data(), d_ltype.size()))) return rc;
+    return upload(s->eng, m.d_types, d_types.data(), d_types.size());
+}
+
 int build_tiles(dsf_structure *s, bool by_type)
 {
     const int n = s->n_atoms;
     s->perm.resize(n);
     std::iota(s->perm.begin(), s->perm.end(), 0);
-    // atoms without anisotropic ADPs first, then by type: a tile holds one ADP kind
+    // atoms without anisotropic ADPs first, then those without l >= 3 populations, then by type: a tile holds one ADP
+    // kind (and of pk_kernel one kind of angular sums)
+    const auto high = [&](int x) { return type_lmax(s, s->atom_type[x], true) >= 3; };
     std::stable_sort(s->perm.begin(), s->perm.end(), [&](int x, int y) {
         const int kx = s->adpk[x] == 6, ky = s->adpk[y] == 6;
         if (kx != ky) return kx < ky;
+        if (by_type && high(x) != high(y)) return high(x) < high(y);
         if (by_type && s->atom_type[x] != s->atom_type[y]) return s->atom_type[x] < s->atom_type[y];
         return false;
     });
@@ -1080,6 +1184,12 @@ int build_tiles(dsf_structure *s, bool by_type)
     if ((rc = upload(e, s->d_anom_f, an_f.data(), an_f.size()))) return rc;
     s->active_host.assign(n, 1);
     if ((rc = upload(e, s->d_active, s->active_host.data(), s->active_host.size()))) return rc;
+    if ((rc = build_pk_map(s, s->pkm[0], by_type, true))) return rc;
+    if ((rc = build_pk_map(s, s->pkm[1], by_type, false))) return rc;
+    // two atoms per thread while the pairs leave at most a fifth of the slots empty: one atom per thread costs about
+    // a quarter more time per atom
+    s->pk_pairs = s->pkm[0].used <= 1.2 * n;
+    if (s->model != MODEL_HC && (rc = upload_pk_info(s))) return rc;  // HC: with the populations (compute_global_plm)
     // per-atom buffers
     DSF_CUDA(s->d_xq.alloc(12 * (size_t)n));
     DSF_CUDA(s->d_xlo.alloc(12 * (size_t)n));
@@ -1105,15 +1215,18 @@ int ensure_tables(dsf_structure *s, bool fp64, bool mp)
     const int p = fp64 ? 1 : 0;
     const size_t esz = fp64 ? sizeof(double) : sizeof(float);
     const size_t row = 8 * (size_t)s->n_hkl_pad * std::max(1, s->n_types);
-    const bool pk = pk_form_compiled(s, fp64);
-    const bool built = (pk ? !s->pk_ok : !s->rs_ok[p]) || !s->tr_ok[p] || (mp && !s->trm_ok[p]);
-    if (pk && !s->pk_ok) {
-        const size_t rec = pk_rec_bytes<double>(s->model == MODEL_HC, s->n_sym, s->n_sym / s->pk.cs);
-        DSF_CUDA(s->d_pk_d.alloc(rec * (size_t)s->n_hkl_pad));
-        DSF_CUDA(launch_pk_prep(s->dev, s->n_hkl_pad, s->pk.cs, 2, s->d_pk_d.p, e->setup));
-        s->pk_ok = true;
+    const int pk = pk_kind(s, fp64, mp);
+    const bool built = (pk >= 0 ? !s->pk_ok[pk] : !s->rs_ok[p]) || !s->tr_ok[p] || (mp && !s->trm_ok[p]);
+    if (pk >= 0 && !s->pk_ok[pk]) {
+        const bool hc = s->model == MODEL_HC;
+        const int nc = s->n_sym / s->pk.cs;
+        const size_t rec = pk == 1 ? pk_rec_bytes<float>(hc, s->n_sym, nc) : pk_rec_bytes<double>(hc, s->n_sym, nc);
+        static_assert(sizeof(F2) == sizeof(double), "two-atom records have the FP64 records' size");
+        DSF_CUDA(s->d_pk[pk].alloc(rec * (size_t)s->n_hkl_pad));
+        DSF_CUDA(launch_pk_prep(s->dev, s->n_hkl_pad, s->pk.cs, pk, s->d_pk[pk].p, e->setup));
+        s->pk_ok[pk] = true;
     }
-    if (!pk && !s->rs_ok[p]) {
+    if (pk < 0 && !s->rs_ok[p]) {
         DevBuf &rs = fp64 ? s->d_rs_d : s->d_rs_f;
         DSF_CUDA(rs.alloc(rs_record_bytes(fp64) * (size_t)s->n_hkl_pad * s->n_sym));
         DSF_CUDA(launch_rs_prep(s->dev, s->n_hkl_pad, fp64 ? nullptr : rs.p, fp64 ? rs.p : nullptr, e->setup));
@@ -1767,7 +1880,8 @@ int dsf_structure_destroy(dsf_structure *s)
                       &s->d_dtdf, &s->d_gw_d, &s->d_gw_f, &s->d_facc, &s->d_gacc, &s->d_out, &s->d_plm_lmax,
                       &s->d_rs_f, &s->d_rs_d, &s->d_tr_f, &s->d_tr_d, &s->d_trm_f, &s->d_trm_d, &s->d_err,
                       &s->d_hperm, &s->d_cont, &s->d_tile_lmax, &s->d_lcs, &s->d_type_plm, &s->d_type_lmax,
-                      &s->d_atom_type0, &s->d_step_f, &s->d_step_d, &s->d_pk_d};
+                      &s->d_atom_type0, &s->d_step_f, &s->d_step_d, &s->d_pk[0], &s->d_pk[1], &s->d_pk[2], &s->pkm[0].d_slot, &s->pkm[0].d_ltype, &s->pkm[0].d_info,
+                      &s->pkm[0].d_types, &s->pkm[1].d_slot, &s->pkm[1].d_ltype, &s->pkm[1].d_info, &s->pkm[1].d_types};
     for (DevBuf *b : bufs) b->release();
     if (s->ev_begin) cudaEventDestroy(s->ev_begin);
     if (s->ev_end) cudaEventDestroy(s->ev_end);
@@ -1792,7 +1906,7 @@ int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl)
         s->n_hkl_pad = 0;
         s->have_hkl = true;
         for (int p = 0; p < 2; p++) s->rs_ok[p] = s->tr_ok[p] = s->trm_ok[p] = false;
-        s->pk_ok = false;
+        for (bool &ok : s->pk_ok) ok = false;
         refresh_dev(s);
         return DSF_OK;
     }
@@ -1814,10 +1928,14 @@ int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl)
         s->hperm.resize(n_hkl);
         for (int i = 0; i < n_hkl; i++) s->hperm[i] = key[i].second;
     }
+    // cont: 1 where a reflection takes its phases from the one before; 0 at line starts and, so that the recurrence's
+    // rounding cannot build up, at every anchor_interval-th reflection of a line (there the phase is exact again)
+    const int anchor = anchor_interval(s->n_sym);
     std::vector<int> cont(n_pad, 0);
-    for (int i = 1; i < n_hkl; i++) {
+    for (int i = 1, run = 0; i < n_hkl; i++) {
         const int *p = hkl + 3 * s->hperm[i - 1], *q = hkl + 3 * s->hperm[i];
-        cont[i] = (p[0] == q[0] && p[1] == q[1] && q[2] == p[2] + 1) ? 1 : 0;
+        run = (p[0] == q[0] && p[1] == q[1] && q[2] == p[2] + 1) ? run + 1 : 0;
+        cont[i] = run % anchor != 0;
     }
     std::vector<int4> h4(n_pad, make_int4(0, 0, 0, 0));
     std::vector<double> h2(n_pad, 0.0), mult(n_pad, 0.0), cinv(2 * (size_t)n_pad, 0.0);
@@ -1870,7 +1988,7 @@ int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl)
     refresh_dev(s);
     // resident per-(reflection, operation) and radial tables: FP32 now, FP64 on the first FP64 call
     for (int p = 0; p < 2; p++) s->rs_ok[p] = s->tr_ok[p] = s->trm_ok[p] = false;
-    s->pk_ok = false;
+    for (bool &ok : s->pk_ok) ok = false;
     int rc2 = ensure_tables(s, false, false);
     if (rc2) return rc2;
     DSF_CUDA(cudaStreamSynchronize(e->setup));
@@ -1989,7 +2107,8 @@ int64_t dsf_structure_device_bytes(const dsf_structure *s)
                             &s->d_dmat, &s->d_raw, &s->d_dtdf, &s->d_gw_d, &s->d_gw_f, &s->d_facc, &s->d_gacc,
                             &s->d_out, &s->d_plm_lmax, &s->d_rs_f, &s->d_rs_d, &s->d_tr_f, &s->d_tr_d,
                             &s->d_trm_f, &s->d_trm_d, &s->d_err, &s->d_hperm, &s->d_cont, &s->d_tile_lmax,
-                            &s->d_lcs, &s->d_type_plm, &s->d_type_lmax, &s->d_atom_type0, &s->d_step_f, &s->d_step_d, &s->d_pk_d};
+                            &s->d_lcs, &s->d_type_plm, &s->d_type_lmax, &s->d_atom_type0, &s->d_step_f, &s->d_step_d, &s->d_pk[0], &s->d_pk[1], &s->d_pk[2], &s->pkm[0].d_slot, &s->pkm[0].d_ltype, &s->pkm[0].d_info, &s->pkm[0].d_types,
+                            &s->pkm[1].d_slot, &s->pkm[1].d_ltype, &s->pkm[1].d_info, &s->pkm[1].d_types};
     int64_t b = 0;
     for (const DevBuf *p : bufs) b += (int64_t)p->bytes;
     return b;
@@ -2166,17 +2285,15 @@ static std::string tune_key(const dsf_structure *s, bool fp64, bool mp, bool gra
     return k;
 }
 
-// blocks per SM, sub-tile cap and register-capped form of a call: the autotuner's candidate under trial, else the
-// tuned shape of the key, else the rule (75 blocks per SM, the longest sub-tile, the compiler's registers)
-static void call_shape(dsf_structure *s, bool fp64, bool mp, bool grad, int &bps, int &ht, int &occ3)
+// blocks per SM and sub-tile cap of a call: the autotuner's candidate under trial, else the tuned shape of the key,
+// else the rule (75 blocks per SM, the longest sub-tile)
+static void call_shape(dsf_structure *s, bool fp64, bool mp, bool grad, int &bps, int &ht)
 {
     bps = 75;
     ht = 0;
-    occ3 = 0;
     if (s->tune_bps > 0) {
         bps = s->tune_bps;
         ht = s->tune_ht;
-        occ3 = s->tune_occ3;
         return;
     }
     dsf_engine *e = s->eng;
@@ -2185,7 +2302,6 @@ static void call_shape(dsf_structure *s, bool fp64, bool mp, bool grad, int &bps
     if (it != e->tuned.end()) {
         bps = it->second[0];
         ht = it->second[1];
-        occ3 = it->second[2];
     }
 }
 
@@ -2195,64 +2311,93 @@ static bool inv_kernel(const dsf_structure *s, bool fp64)
     return s->inv_pairs && !fp64 && s->model != MODEL_HC && table_count_compiled(s->n_sym);
 }
 
-// one structure's launch of pk_kernel: every tile, reflection chunks that give about `bps` blocks per SM, at least
-// one sub-tile each.  Sub-tiles of 16 reflections where the shared-memory budget allows (two blocks per SM); shorter
-// ones only where the reflections are too few to give every SM its blocks.
-static int launch_pk_structure(dsf_structure *s, bool fp64, bool mp, bool grad, int bps, int ht_cap, cudaStream_t st)
+static const PkMap &pk_map(const dsf_structure *s, int kind)
+{
+    return s->pkm[kind == 0 && s->model == MODEL_HC ? 0 : 1];
+}
+
+// the parts of a pk_kernel launch that do not depend on the grid: buffers, tables, and the sub-tile length: 16
+// reflections where the shared-memory budget of several blocks per SM allows (FP32: four blocks; FP64: two, else one),
+// shorter where a block's share of the reflections (`want`) is shorter
+static int pk_setup(dsf_structure *s, int kind, bool mp, bool grad, int want, int ht_cap, CallBuffers &C, PkLaunch &L,
+                    size_t &smem)
 {
     dsf_engine *e = s->eng;
-    CallBuffers C;
+    const bool fp64 = kind == 2;
     C.gw_d = s->d_gw_d.as<double2>();
     C.gw_f = s->d_gw_f.as<float2>();
     C.f_acc = s->d_facc.as<double2>();
     C.g_acc = s->d_gacc.as<double>();
-    PkLaunch L{};
-    L.max_types = std::max(s->n_tiles_plain > 0 ? s->max_types_plain : 1,
-                           s->n_tiles_plain < s->n_tiles ? s->max_types_aniso : 1);
+    L = PkLaunch{};
+    const PkMap &m = pk_map(s, kind);
+    L.T.slot = m.d_slot.as<int>();
+    L.T.ltype = m.d_ltype.as<int>();
+    L.T.info = m.d_info.as<int4>();
+    L.T.types = m.d_types.as<int>();
+    L.T.n_plain = m.n_plain;
+    L.T.max_types = m.max_types;
     L.n_hkl_pad = s->n_hkl_pad;
-    L.n_plain = s->n_tiles_plain;
-    L.pk = s->d_pk_d.p;
+    L.pk = s->d_pk[kind].p;
     L.tr = fp64 ? s->d_tr_d.p : s->d_tr_f.p;
     L.trm = fp64 ? s->d_trm_d.p : s->d_trm_f.p;
     L.cont = s->d_cont.as<int>();
-    L.tile_lmax = s->d_tile_lmax.as<int>();
     L.math = e->d_math;
     L.error = s->d_err.as<int>();
     L.stall_first = s->debug_stall;
     s->debug_stall = 0;
-    const bool mp_hc = mp && s->model == MODEL_HC, gr = grad || mp_hc || s->model != MODEL_HC;
     const int ncos = s->n_sym / s->pk.cs;
     auto bytes = [&](int ht) {
-        return mp_hc ? pk_smem_bytes<double, true>(s->model, ht, s->n_sym, ncos, L.max_types, true)
-                     : pk_smem_bytes<double, false>(s->model, ht, s->n_sym, ncos, L.max_types, gr);
+        const int md = s->model, n = s->n_sym, mt = m.max_types;
+        if (kind == 0) return pk_smem_bytes<F2, false>(md, ht, n, ncos, mt, grad);
+        if (kind == 1 && !mp) return pk_smem_bytes<float, false>(md, ht, n, ncos, mt, grad);
+        if (kind == 1) return pk_smem_bytes<float, true>(md, ht, n, ncos, mt, true);
+        return mp ? pk_smem_bytes<double, true>(md, ht, n, ncos, mt, true)
+                  : pk_smem_bytes<double, false>(md, ht, n, ncos, mt, grad);
     };
-    const int n_chunks0 = chunk_count(e, s->n_tiles, s->n_hkl, bps);
-    const int want = std::max(1, (s->n_hkl + n_chunks0 - 1) / n_chunks0);
-    // two blocks per SM with sub-tiles of 16 or 8 reflections, else one block with the longest that fits
+    const size_t budget = fp64 || kind == 1 ? 110 * 1024 : 55 * 1024;
     int ht = kMaxHT;
-    if (bytes(8) > 110 * 1024)
+    if (bytes(8) > budget)
         while (ht > 4 && bytes(ht) > e->max_smem) ht /= 2;
-    else if (bytes(ht) > 110 * 1024)
+    else if (bytes(ht) > budget)
         ht = 8;
     while (ht > 4 && want < ht) ht /= 2;
     while (ht_cap >= 4 && ht > ht_cap) ht /= 2;
-    if (bytes(ht) > e->max_smem) return fail(e, DSF_ERR_UNSUPPORTED, "shared-memory tile does not fit this device");
+    smem = bytes(ht);
+    if (smem > e->max_smem) return fail(e, DSF_ERR_UNSUPPORTED, "shared-memory tile does not fit this device");
     L.ht = ht;
-    L.hkl_chunk = (want + ht - 1) / ht * ht;
+    return DSF_OK;
+}
+
+// one structure's launch of pk_kernel: every tile, reflection chunks that give about `bps` blocks per SM
+static int launch_pk_structure(dsf_structure *s, int kind, bool mp, bool grad, int bps, int ht_cap, cudaStream_t st)
+{
+    dsf_engine *e = s->eng;
+    CallBuffers C;
+    PkLaunch L;
     PkArgs A;
+    const int n_tiles = pk_map(s, kind).n_tiles;
+    const int n_chunks0 = chunk_count(e, n_tiles, s->n_hkl, bps);
+    const int want = std::max(1, (s->n_hkl + n_chunks0 - 1) / n_chunks0);
+    const bool hc = s->model == MODEL_HC;
+    mp = mp && hc;
+    int rc = pk_setup(s, kind, mp, grad || !hc, want, ht_cap, C, L, A.smem);
+    if (rc) return rc;
+    L.hkl_chunk = (want + L.ht - 1) / L.ht * L.ht;
     A.S = &s->dev;
     A.C = &C;
     A.L = &L;
     A.form = s->pk;
-    A.n_tiles = s->n_tiles;
+    A.n_tiles = n_tiles;
     A.n_chunks = (s->n_hkl + L.hkl_chunk - 1) / L.hkl_chunk;
-    A.smem = bytes(ht);
     A.st = st;
-    if (s->model == MODEL_IAM) DSF_CUDA(launch_pk_f64_iam(A));
-    else if (s->model == MODEL_TABLE) DSF_CUDA(launch_pk_f64_table(A));
-    else if (mp_hc) DSF_CUDA(launch_pk_f64_hc_mp(A));
-    else if (grad) DSF_CUDA(launch_pk_f64_hc(A));
-    else DSF_CUDA(launch_pk_f64_hc_f(A));
+    A.split_kinds = (long long)A.n_tiles * A.n_chunks >= 16ll * e->n_sm;
+    cudaError_t ce;
+    if (s->model == MODEL_IAM) ce = kind == 2 ? launch_pk_f64_iam(A) : launch_pk_f32_iam(A);
+    else if (s->model == MODEL_TABLE) ce = launch_pk_f64_table(A);
+    else if (mp) ce = kind == 2 ? launch_pk_f64_hc_mp(A) : launch_pk_f32_hc_mp(A);
+    else if (grad) ce = kind == 2 ? launch_pk_f64_hc(A) : kind == 1 ? launch_pk_f32_hc1(A) : launch_pk_f32_hc(A);
+    else ce = kind == 2 ? launch_pk_f64_hc_f(A) : kind == 1 ? launch_pk_f32_hc1_f(A) : launch_pk_f32_hc_f(A);
+    DSF_CUDA(ce);
     return DSF_OK;
 }
 
@@ -2291,23 +2436,23 @@ int dsf_calculate_device(dsf_structure *s, int precision, int flags, const doubl
     CallBuffers C;
     SfLaunch L;
     SignTable G;
-    const bool pk = pk_form_compiled(s, fp64);
-    if (!pk) call_buffers(s, fp64, C, L, G);
+    const int pk = pk_kind(s, fp64, mp);
+    if (pk < 0) call_buffers(s, fp64, C, L, G);
     if (!s->ev_begin) {
         DSF_CUDA(cudaEventCreate(&s->ev_begin));
         DSF_CUDA(cudaEventCreate(&s->ev_end));
     }
     const bool grad = (flags & (DSF_D_XYZ | DSF_D_ADP | DSF_D_OCC | DSF_D_MULTIPOLE)) != 0;
-    int bps, ht_cap, occ3;
-    call_shape(s, fp64, mp, grad, bps, ht_cap, occ3);
+    int bps, ht_cap;
+    call_shape(s, fp64, mp, grad, bps, ht_cap);
     DSF_CUDA(cudaEventRecord(s->ev_begin, st));
-    if (pk) {
-        if ((rc = launch_pk_structure(s, fp64, mp, grad, bps, ht_cap, st))) return rc;
+    if (pk >= 0) {
+        if ((rc = launch_pk_structure(s, pk, mp, grad, bps, ht_cap, st))) return rc;
         launches++;
     }
     // one launch per ADP kind (tiles [0, n_tiles_plain) without anisotropic ADPs), reflection chunks of
     // chunk_count
-    for (int kind = 0; kind < 2 && !pk; kind++) {
+    for (int kind = 0; kind < 2 && pk < 0; kind++) {
         int nt, n_chunks;
         size_t smem;
         const int ntk = kind ? s->n_tiles - s->n_tiles_plain : s->n_tiles_plain;
@@ -2329,7 +2474,6 @@ int dsf_calculate_device(dsf_structure *s, int precision, int flags, const doubl
         A.st = st;
         A.grad = grad;
         A.inv = inv_kernel(s, fp64);
-        A.occ3 = occ3 != 0;
         DSF_CUDA(launch_sf3(A, s->model, fp64, mp, kind == 1));
         launches++;
     }
@@ -2372,12 +2516,11 @@ int dsf_autotune(dsf_structure *s, int precision, int flags, int *blocks_per_sm,
         out.d_kappa_prime = p;
     }
     int rc = DSF_OK;
-    auto timed = [&](int bps, int cap, int occ3, double &ms) {
+    auto timed = [&](int bps, int cap, double &ms) {
         s->tune_bps = bps;
         s->tune_ht = cap;
-        s->tune_occ3 = occ3;
         rc = dsf_calculate_device(s, precision, flags, buf, &out, e->stream);
-        s->tune_bps = s->tune_ht = s->tune_occ3 = 0;
+        s->tune_bps = s->tune_ht = 0;
         if (rc) return false;
         if (cudaStreamSynchronize(e->stream) != cudaSuccess) {
             rc = fail(e, DSF_ERR_CUDA, "autotune call failed");
@@ -2387,38 +2530,34 @@ int dsf_autotune(dsf_structure *s, int precision, int flags, int *blocks_per_sm,
         return ms >= 0;
     };
     double warm = 0, best = 1e300;
-    int best_bps = 75, best_cap = 0, best_occ3 = 0;
-    // the register-capped form exists for the FP32 multipole-adjoint kernels
-    const int n_occ = (s->model == MODEL_HC && mp && !fp64) ? 2 : 1;
-    if (timed(75, 0, 0, warm)) {
+    int best_bps = 75, best_cap = 0;
+    if (timed(75, 0, warm)) {
         const int reps = warm < 20.0 ? 3 : 1;
-        for (int occ3 = 0; occ3 < n_occ && !rc; occ3++)
-            for (const int bps : {24, 48, 75, 150})
-                for (const int cap : {0, 8}) {
-                    double t = 1e300;
-                    for (int r = 0; r < reps; r++) {
-                        double ms;
-                        if (!timed(bps, cap, occ3, ms)) break;
-                        t = std::min(t, ms);
-                    }
-                    if (rc) break;
-                    if (t < best) {
-                        best = t;
-                        best_bps = bps;
-                        best_cap = cap;
-                        best_occ3 = occ3;
-                    }
+        for (const int bps : {24, 48, 75, 150})
+            for (const int cap : {0, 8}) {
+                double t = 1e300;
+                for (int r = 0; r < reps; r++) {
+                    double ms;
+                    if (!timed(bps, cap, ms)) break;
+                    t = std::min(t, ms);
                 }
+                if (rc) break;
+                if (t < best) {
+                    best = t;
+                    best_bps = bps;
+                    best_cap = cap;
+                }
+            }
     }
     cudaFree(buf);
     if (rc) return rc;
     {
         std::lock_guard<std::mutex> lock(e->tune_mtx);
-        e->tuned[tune_key(s, fp64, mp, grad)] = {best_bps, best_cap, best_occ3};
+        e->tuned[tune_key(s, fp64, mp, grad)] = {best_bps, best_cap, 0};
     }
     if (blocks_per_sm) *blocks_per_sm = best_bps;
     if (ht) *ht = best_cap;
-    if (occupancy) *occupancy = best_occ3 ? 3 : 0;
+    if (occupancy) *occupancy = 0;
     if (best_ms) *best_ms = best;
     return DSF_OK;
 }
@@ -2438,7 +2577,7 @@ int dsf_tuning_lookup(dsf_structure *s, int precision, int flags, int *blocks_pe
     const bool hit = it != e->tuned.end();
     if (blocks_per_sm) *blocks_per_sm = hit ? it->second[0] : 75;
     if (ht) *ht = hit ? it->second[1] : 0;
-    if (occupancy) *occupancy = (hit && it->second[2]) ? 3 : 0;
+    if (occupancy) *occupancy = 0;
     if (tuned) *tuned = hit ? 1 : 0;
     return DSF_OK;
 }
@@ -2456,7 +2595,8 @@ int dsf_tuning_save(dsf_engine *e, const char *path)
     return DSF_OK;
 }
 
-// adds the shapes of a file written by dsf_tuning_save (keys name the device's SM count, so shapes tuned on
+// adds the shapes of a file written by dsf_tuning_save (the third number, once a register-capped form, is read and
+// not used; keys name the device's SM count, so shapes tuned on
 // another kind of device are never matched)
 int dsf_tuning_load(dsf_engine *e, const char *path)
 {
@@ -2467,7 +2607,7 @@ int dsf_tuning_load(dsf_engine *e, const char *path)
     int bps, ht, occ3;
     std::lock_guard<std::mutex> lock(e->tune_mtx);
     while (std::fscanf(f, "%159s %d %d %d", key, &bps, &ht, &occ3) == 4)
-        if (bps > 0 && bps <= 4096 && ht >= 0 && ht <= kMaxHT && (occ3 == 0 || occ3 == 1)) e->tuned[key] = {bps, ht, occ3};
+        if (bps > 0 && bps <= 4096 && ht >= 0 && ht <= kMaxHT && (occ3 == 0 || occ3 == 1)) e->tuned[key] = {bps, ht, 0};
     std::fclose(f);
     return DSF_OK;
 }
@@ -2578,13 +2718,36 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
         std::vector<SfBatchItem> items;
     };
     std::vector<Group> groups;
+    struct PkGroup {
+        int model, kind;
+        PkForm form;
+        std::vector<dsf_structure *> items;
+    };
+    std::vector<PkGroup> pk_groups;  // FP32 HC and IAM structures: pk_batch_kernel, both ADP kinds in one launch
     for (int i = 0; i < n; i++) {
         dsf_structure *s = structures[i];
         const bool mp = (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC;
-        if (pk_form_compiled(s, fp64)) {
+        const int pk = pk_kind(s, fp64, mp);
+        if (pk == 2 || (pk == 1 && mp)) {
             const bool grad = (flags & (DSF_D_XYZ | DSF_D_ADP | DSF_D_OCC | DSF_D_MULTIPOLE)) != 0;
-            if ((rc = launch_pk_structure(s, fp64, mp, grad, 75, 0, st))) return rc;
+            if ((rc = launch_pk_structure(s, pk, mp, grad, 75, 0, st))) return rc;
             launches++;
+            continue;
+        }
+        if (pk >= 0) {
+            PkGroup *g = nullptr;
+            for (auto &x : pk_groups)
+                if (x.model == s->model && x.kind == pk && x.form.n_sym == s->pk.n_sym && x.form.cs == s->pk.cs &&
+                    x.form.pat == s->pk.pat && x.form.inv == s->pk.inv)
+                    g = &x;
+            if (!g) {
+                pk_groups.emplace_back();
+                g = &pk_groups.back();
+                g->model = s->model;
+                g->kind = pk;
+                g->form = s->pk;
+            }
+            g->items.push_back(s);
             continue;
         }
         CallBuffers C;
@@ -2692,6 +2855,39 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
             A.smem = g.smem;
             A.st = (lane++ & 1) ? e->side : st;
             DSF_CUDA(launch_k3b_f32(A, g.model, g.aniso == 1));
+            launches++;
+        }
+    static PkBatch PKB;  // host staging of the launch parameters, under the same lock
+    for (auto &g : pk_groups)
+        for (size_t b0 = 0; b0 < g.items.size(); b0 += kBatchItems) {
+            const int m = (int)std::min<size_t>(kBatchItems, g.items.size() - b0);
+            PKB.n = m;
+            double pairs = 0;
+            for (int k = 0; k < m; k++) pairs += (double)pk_map(g.items[b0 + k], g.kind).n_tiles * g.items[b0 + k]->n_hkl;
+            const int want = (int)std::max(64.0, pairs / (std::max(1, e->n_sm) * 24.0));
+            int blocks = 0;
+            PkArgs A;
+            for (int k = 0; k < m; k++) {
+                dsf_structure *s = g.items[b0 + k];
+                PkBatchItem &it = PKB.item[k];
+                size_t smem;
+                if ((rc = pk_setup(s, g.kind, false, true, std::min(want, s->n_hkl), 0, it.C, it.L, smem))) return rc;
+                it.S = s->dev;
+                it.n_tiles = pk_map(s, g.kind).n_tiles;
+                const int chunk = std::min(want, s->n_hkl);
+                it.L.hkl_chunk = (chunk + it.L.ht - 1) / it.L.ht * it.L.ht;
+                PKB.block_begin[k] = blocks;
+                blocks += it.n_tiles * ((s->n_hkl + it.L.hkl_chunk - 1) / it.L.hkl_chunk);
+                A.smem = std::max(A.smem, smem);
+            }
+            PKB.block_begin[m] = blocks;
+            A.B = &PKB;
+            A.form = g.form;
+            A.blocks = blocks;
+            A.st = (lane++ & 1) ? e->side : st;
+            DSF_CUDA(g.model != MODEL_HC ? launch_pk_f32_iam_batch(A)
+                     : g.kind == 1       ? launch_pk_f32_hc1_batch(A)
+                                         : launch_pk_f32_hc_batch(A));
             launches++;
         }
     DSF_CUDA(cudaEventRecord(e->ev_join, e->side));

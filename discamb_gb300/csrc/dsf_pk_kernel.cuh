@@ -8,7 +8,14 @@
 //   FP32: the FMA pipe and instruction issue.  A packed instruction (fma.f32x2) does two atoms in one issue slot
 //     and holds the FMA pipe for two cycles, so the packed form halves the issue slots of everything that is the
 //     same for both atoms: arithmetic, shared-memory reads of the reflection record (stored duplicated, {y, y}),
-//     the reduction of F over the warp, loop and barrier work.
+//     the reduction of F over the warp, loop and barrier work.  The code is kept in straight stretches: tiles with
+//     and without l = 3, 4 harmonics run their own copy, and a group of four reflections without a line start runs
+//     without a branch.  Against sf_grad_body (the same box): 5,000 isotropic atoms, P2_1 2_1 2_1, 54,704
+//     reflections 1.70 -> 1.48 ms (189 warp instructions per two atoms and reflection instead of 2 x 167; the FMA
+//     pipe 60% busy, two warps per scheduler); structure factors of 8,000 atoms, 100,003 reflections 4.10 -> 3.29 ms;
+//     50,000 atoms, P4_3 2_1 2, multipole adjoint (V = float) 369 -> 292 ms; independent atoms, P2_1/c, 2,000 atoms,
+//     50,021 reflections 0.47 -> 0.27 ms (one form factor for all operations: the transform of the phases alone, and
+//     of an inversion pair only its real or imaginary half).
 //   FP64: the FP64 pipe (about 1.6 lanes per clock and SM, 1/75 of FP32), so only the number of FP64 instructions
 //     counts; integer work, shared-memory tables and loads are free beside it.  Exponentials and sines come from
 //     shared-memory tables plus a short polynomial (exp_tab, sincos_tab), phases are exact 64-bit fixed point, and
@@ -149,6 +156,39 @@ __device__ __forceinline__ double widen(float f)
     return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
 }
 
+// FP32: sincos_fixed (sf_kernel.cuh) for every atom of the thread: P the phase in 2^32 fixed point per atom, lo the
+// remainder in turns; the polynomials as packed operations
+template <typename V>
+__device__ __forceinline__ void sincos_fixed_v(const uint32_t (&P)[VTraits<V>::NA], V lo, V *sn, V *cs)
+{
+    constexpr int NA = VTraits<V>::NA;
+    uint32_t q[NA];
+    V r;
+#pragma unroll
+    for (int k = 0; k < NA; k++) {
+        q[k] = (P[k] + 0x20000000u) >> 30;
+        vput(r, k, (float)(int32_t)(P[k] - (q[k] << 30)));
+    }
+    const V th = vfma(r, vdup<V>(1.4629180792671596e-09f), vmul(vdup<V>(6.283185307179586f), lo));
+    const V t2 = vmul(th, th);
+    V sp = vfma(t2, vdup<V>(2.7557319e-06f), vdup<V>(-1.9841270e-04f));
+    sp = vfma(t2, sp, vdup<V>(8.3333333e-03f));
+    sp = vfma(t2, sp, vdup<V>(-1.6666667e-01f));
+    const V sv = vfma(vmul(th, t2), sp, th);
+    V cp = vfma(t2, vdup<V>(2.4801587e-05f), vdup<V>(-1.3888889e-03f));
+    cp = vfma(t2, cp, vdup<V>(4.1666668e-02f));
+    cp = vfma(t2, cp, vdup<V>(-0.5f));
+    const V cv = vfma(t2, cp, vdup<V>(1.0f));
+#pragma unroll
+    for (int k = 0; k < NA; k++) {
+        const float s1 = vget(sv, k), c1 = vget(cv, k);
+        const float ss = (q[k] & 1u) ? c1 : s1, cc = (q[k] & 1u) ? s1 : c1;
+        // the quadrant's signs on the sign bits
+        vput(*sn, k, __uint_as_float(__float_as_uint(ss) ^ ((q[k] & 2u) << 30)));
+        vput(*cs, k, __uint_as_float(__float_as_uint(cc) ^ (((q[k] + 1u) & 2u) << 30)));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // reflection records
 // ---------------------------------------------------------------------------
@@ -227,8 +267,11 @@ __device__ __forceinline__ void pk_wht(const V (&u)[CS], V (&W)[CS])
 template <typename V>
 __host__ __device__ constexpr int pk_threads() { return kTileAtoms / VTraits<V>::NA; }
 // line steps (and FP64 populations) in shared memory instead of registers
-template <typename V, bool MP, int NSC>
-__host__ __device__ constexpr bool pk_step_smem() { return NSC >= 8 || (sizeof(V) == 8 && VTraits<V>::NA == 1 && MP); }
+template <typename V, bool MP, bool ANISO, int NSC>
+__host__ __device__ constexpr bool pk_step_smem()
+{
+    return NSC >= 8 || (VTraits<V>::NA == 2 ? ANISO && NSC >= 4 : sizeof(V) == 8 && MP);
+}
 
 template <typename V>
 struct PkStage {
@@ -258,22 +301,43 @@ __host__ __device__ inline size_t pk_smem_bytes(int model, int ht, int nsc, int 
     b += sizeof(R) * 2 * (size_t)(pk_threads<V>() / 32) * ht;
     if (grad) b += sizeof(R) * 2 * (size_t)n_channels<R, MP>() * kTileAtoms;
     b += sizeof(int) * kMaxTileTypes;
-    if (sizeof(R) == 8) b += sizeof(double) * kMathTab;
-    if (nsc >= 8 || (sizeof(R) == 8 && MP)) b += 2 * sizeof(V) * (size_t)nsc * pk_threads<V>();
+    b += sizeof(R) == 8 ? sizeof(double) * kMathTab : 32 * (size_t)kTileAtoms;
+    if (nsc >= 8 || (VTraits<V>::NA == 2 ? nsc >= 4 : sizeof(R) == 8 && MP)) b += 2 * sizeof(V) * (size_t)nsc * pk_threads<V>();
     if (sizeof(R) == 8 && hc) b += sizeof(V) * 25 * (size_t)pk_threads<V>();
     return b;
 }
 
+// The tiles of a structure for pk_kernel: kTileAtoms slots each, of atoms of one ADP kind, sorted so that a tile holds
+// atoms with l >= 3 populations or none, and few types.  Two forms: dense, and (two atoms per thread, HC) pairs of
+// slots 2t, 2t + 1 with atoms of one type each, a type with an odd count leaving one slot empty, so that a thread's
+// two atoms share their radial terms.
+struct PkTiles {
+    const int *slot;    // [n_tiles][kTileAtoms] sorted atom index, -1: empty
+    const int *ltype;   // [n_tiles][kTileAtoms] local type
+    const int4 *info;   // [n_tiles] slots in use, types, highest l of the populations that are not zero, of all of them
+    const int *types;   // [n_tiles][kMaxTileTypes]
+    int n_plain;        // tiles below it hold atoms without anisotropic ADPs
+    int max_types;
+};
+
+struct PkYes {
+    static constexpr bool value = true;
+};
+struct PkNo {
+    static constexpr bool value = false;
+};
+
 struct PkLaunch {
-    int hkl_chunk, ht, max_types, n_hkl_pad, n_plain;  // n_plain: tiles below it hold atoms without anisotropic ADPs
+    int hkl_chunk, ht, n_hkl_pad;
+    PkTiles T;
     const void *pk;        // reflection records
     const void *tr, *trm;  // R [n_types][n_hkl_pad][8]
-    const int *cont, *tile_lmax;
+    const int *cont;
     const double *math;    // kMathTab doubles (FP64)
     int *error, stall_first;
 };
 
-template <typename V, int MODEL, bool MP, bool ANISO, int NSC, int CS, bool GRAD, bool INV, int PAT>
+template <typename V, int MODEL, bool MP, bool ANISO, int NSC, int CS, bool GRAD, bool INV, int PAT, bool ROLL, bool HL>
 __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers &C, const PkLaunch &L, const int tile,
                                         const int chunk)
 {
@@ -286,12 +350,14 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     constexpr int NC = NSC / CS, NZ = INV ? NSC / 2 : NSC;
     constexpr bool INVC = INV && CS == NSC && CS > 1;  // the images lie in the same coset
     constexpr int NT = n_channels<R, MP>();
+    constexpr int NL = HL ? 5 : 3, NH = NL * NL;  // levels of the angular sums (HL: l = 3, 4 too), harmonics
+    constexpr bool SAME = HC && NA == 2;          // a thread's atoms share their type
     constexpr int TH = pk_threads<V>(), WARPS = TH / 32;
-    constexpr bool STEP_SM = pk_step_smem<V, MP, NSC>(), PG_SM = F64 && HC;
+    constexpr bool STEP_SM = pk_step_smem<V, MP, ANISO, NSC>(), PG_SM = F64 && HC;
     constexpr int SLOTS = pk_slots<V>(HC);
     constexpr size_t REC = pk_rec_bytes<V>(HC, NSC, NC);
     constexpr int HOFF = HC ? 25 : 0;
-    constexpr bool ROLL_J = NSC > 4 || MP || F64;
+        constexpr bool ROLL_J = NSC > 4 || MP || F64 || ROLL;
     static_assert(NSC % CS == 0 && (CS == 1 || CS == 2 || CS == 4), "cosets of one, two or four");
     static_assert(!INV || (!HC && NSC % 2 == 0), "inversion pairs: generic models");
     static_assert(GRAD || !MP, "the multipole adjoint needs the derivative pass");
@@ -302,13 +368,12 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     const int h_begin = chunk * L.hkl_chunk;
     const int h_end = min(S.n_hkl, h_begin + L.hkl_chunk);
     if (h_begin >= h_end) return;
-    const int a_begin = S.tile_begin[tile], n_at = S.tile_begin[tile + 1] - a_begin;
-    const int nT = S.tile_ntypes[tile];
+    const int4 info = L.T.info[tile];
+    const int n_at = info.x, nT = info.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool high_l = HC && L.tile_lmax[tile] >= 3;
 
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw);
-    const PkStage<V> SL(ht, REC, L.max_types, MP, TABLE);
+    const PkStage<V> SL(ht, REC, L.T.max_types, MP, TABLE);
     unsigned char *stage0 = smem_raw + 64;
     R2 *sF = reinterpret_cast<R2 *>(stage0 + 2 * SL.bytes);  // [WARPS][ht]
     R *sTot = reinterpret_cast<R *>(sF + WARPS * ht);        // [NT][kTileAtoms], Kahan total and compensation
@@ -320,6 +385,9 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     if constexpr (STEP_SM) sp += 2 * sizeof(V) * NSC * TH;
     V *sPg = reinterpret_cast<V *>(sp);    // [25][TH]
     if constexpr (PG_SM) sp += sizeof(V) * 25 * TH;
+    int4 *sX = reinterpret_cast<int4 *>(sp);  // FP32: fixed-point positions and their remainders (read at anchors)
+    float4 *sXl = reinterpret_cast<float4 *>(sX + kTileAtoms);
+    if constexpr (!F64) sp += 32 * kTileAtoms;
     int *sTypes = reinterpret_cast<int *>(sp);
 
     // Small tiles: the block's threads in `split` parts of TH / split atom slots (whole warps), each part taking its
@@ -329,7 +397,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     const int split = TH / slots, part_id = tid / slots, slot = tid - part_id * slots;
     const int seg = ht / split, seg0 = part_id * seg;  // this thread's reflections of a sub-tile: [seg0, seg0 + seg)
 
-    for (int i = tid; i < nT; i += TH) sTypes[i] = S.tile_types[tile * kMaxTileTypes + i];
+    for (int i = tid; i < nT; i += TH) sTypes[i] = L.T.types[tile * kMaxTileTypes + i];
     if constexpr (GRAD) {
         for (int q = tid; q < NT * kTileAtoms; q += TH) {
             sTot[q] = R(0);
@@ -341,7 +409,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     }
     if constexpr (!TABLE) {
         for (int q = tid; q < 2 * (int)(SL.row / 16); q += TH) {  // the zero rows of both stages
-            unsigned char *st = stage0 + (q & 1) * SL.bytes + SL.row * L.max_types;
+            unsigned char *st = stage0 + (q & 1) * SL.bytes + SL.row * L.T.max_types;
             reinterpret_cast<int4 *>(st + SL.tr)[q >> 1] = make_int4(0, 0, 0, 0);
             if constexpr (MP) reinterpret_cast<int4 *>(st + SL.trm)[q >> 1] = make_int4(0, 0, 0, 0);
         }
@@ -391,15 +459,14 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     if (warp == 0 && !L.stall_first) issue(0, h_begin);
 
     // the thread's atoms; absent and excluded ones are all zeros (their radial rows too), so they add nothing
-    V w = vdup<V>(R(0)), anre = w, anim = w, pg[HC && !PG_SM ? 25 : 1], adp[ANISO ? 6 : 1];
+    V w = vdup<V>(R(0)), anre = w, anim = w, pg[HC && !PG_SM ? NH : 1], adp[ANISO ? 6 : 1];
     V step_re[STEP_SM ? 1 : NZ], step_im[STEP_SM ? 1 : NZ], e_re[NZ], e_im[NZ];
-    uint32_t xq[F64 ? 1 : NA][3];
-    float xl[F64 ? 1 : NA][3];
     uint64_t xq64[3] = {0, 0, 0};
-    size_t toff[NA];  // offset of the atom's radial rows inside a stage's table
+    int atom[NA];
+    uint32_t toff[SAME ? 1 : NA];  // offset of the atom's radial rows inside a stage's table
     bool active[NA];
 #pragma unroll
-    for (int q = 0; q < (HC && !PG_SM ? 25 : 1); q++) pg[q] = vdup<V>(R(0));
+    for (int q = 0; q < (HC && !PG_SM ? NH : 1); q++) pg[q] = vdup<V>(R(0));
 #pragma unroll
     for (int q = 0; q < (ANISO ? 6 : 1); q++) adp[q] = vdup<V>(R(0));
 #pragma unroll
@@ -410,18 +477,16 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
 #pragma unroll
     for (int k = 0; k < NA; k++) {
         const int la = slot * NA + k;
-        const size_t a = (size_t)a_begin + la;
-        active[k] = la < n_at && S.atom_active[la < n_at ? a : a_begin] != 0;
-        toff[k] = SL.row * (size_t)L.max_types;
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            if constexpr (!F64) {
-                xq[k][j] = 0;
-                xl[k][j] = 0.f;
-            }
+        atom[k] = la < n_at ? L.T.slot[tile * kTileAtoms + la] : -1;
+        const size_t a = (size_t)max(atom[k], 0);
+        active[k] = atom[k] >= 0 && S.atom_active[a] != 0;
+        if (!SAME || k == 0) toff[SAME ? 0 : k] = (uint32_t)SL.row * L.T.max_types;
+        if constexpr (!F64) {
+            sX[k * TH + tid] = make_int4(0, 0, 0, 0);
+            sXl[k * TH + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if constexpr (PG_SM)
-            for (int q = 0; q < 25; q++) sPg[q * TH + tid] = active[k] ? S.atom_pg_d[25 * a + q] : 0.0;
+            for (int q = 0; q < NH; q++) sPg[q * TH + tid] = active[k] ? S.atom_pg_d[25 * a + q] : 0.0;
         if constexpr (STEP_SM)
             for (int s = 0; s < NSC; s++) {
                 R2 st;
@@ -436,7 +501,8 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
             }
         if (!active[k]) continue;
         any = true;
-        if constexpr (!TABLE) toff[k] = SL.row * (size_t)S.atom_ltype[a];
+        // (an excluded partner of a pair keeps zero populations, weight and dispersion, so the shared rows add nothing)
+        if constexpr (!TABLE) toff[SAME ? 0 : k] = (uint32_t)SL.row * L.T.ltype[tile * kTileAtoms + la];
         if constexpr (F64) {
             w = S.atom_w_d[a];
             const double2 an = S.atom_anom_d[a];
@@ -456,14 +522,11 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
             vput(anim, k, an.y);
 #pragma unroll
             for (int q = 0; q < (ANISO ? 6 : 1); q++) vput(adp[q], k, -S.atom_adp_f[6 * a + q]);
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                xq[k][j] = S.atom_xq[3 * a + j];
-                xl[k][j] = S.atom_xlo[3 * a + j];
-            }
+            sX[k * TH + tid] = make_int4((int)S.atom_xq[3 * a], (int)S.atom_xq[3 * a + 1], (int)S.atom_xq[3 * a + 2], 0);
+            sXl[k * TH + tid] = make_float4(S.atom_xlo[3 * a], S.atom_xlo[3 * a + 1], S.atom_xlo[3 * a + 2], 0.f);
             if constexpr (HC) {
 #pragma unroll
-                for (int q = 0; q < 25; q++) vput(pg[q], k, S.atom_pg_f[25 * a + q]);
+                for (int q = 0; q < NH; q++) vput(pg[q], k, S.atom_pg_f[25 * a + q]);
             }
         }
         if constexpr (!STEP_SM) {
@@ -491,6 +554,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
         const uint32_t phase = parity[buf];
         const bool ok = mbar_wait(&bar[buf], phase);
         parity[buf] ^= 1u;
+        // (the barrier also keeps the block's warps at the same code: without it they run 2% slower)
         if (__syncthreads_or(!ok)) {
             if (tid == 0) {
                 atomicOr(L.error, 1);
@@ -505,13 +569,15 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
         const R *sH2 = reinterpret_cast<const R *>(st + SL.h2);
         const int *sCont = reinterpret_cast<const int *>(st + SL.cont);
 
+        // the first reflection of a stretch: with several parts each stretch is apart from the one before
+        const bool fresh = split > 1 || k_sub == 0;
         // reflection hl of the sub-tile: its partial F over the thread's atoms in (fr, fi)
-        auto reflection = [&](const int hl, R &fr_out, R &fi_out) {
+        auto reflection = [&](const int hl, auto may_anchor, R &fr_out, R &fi_out) {
             const unsigned char *rec = st + SL.rs + REC * (size_t)hl;
             const PkOp *ops = reinterpret_cast<const PkOp *>(rec);
             const V *cos_rec = reinterpret_cast<const V *>(rec + sizeof(PkOp) * NSC);
             // ---- phases: exact at line and stretch starts, one complex multiplication per operation in between
-            if (sCont[hl] == 0 || hl == seg0) {
+            if (decltype(may_anchor)::value && (sCont[hl] == 0 || (hl == seg0 && fresh))) {
 #pragma unroll
                 for (int s = 0; s < NZ; s++) {
                     const PkOp op = ops[s];
@@ -520,15 +586,20 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                                            (uint64_t)(int64_t)op.h[2] * xq64[2] + op.tq;
                         sincos_tab(P, sMath + kExpN, &e_im[s], &e_re[s]);
                     } else {
+                        uint32_t P[NA];
+                        V lo;
 #pragma unroll
                         for (int k = 0; k < NA; k++) {
-                            const uint32_t P = (uint32_t)op.h[0] * xq[k][0] + (uint32_t)op.h[1] * xq[k][1] +
-                                               (uint32_t)op.h[2] * xq[k][2] + (uint32_t)op.h[3];
-                            float sn, cs;
-                            sincos_fixed(P, op.hf[0] * xl[k][0] + op.hf[1] * xl[k][1] + op.hf[2] * xl[k][2], &sn, &cs);
-                            vput(e_re[s], k, cs);
-                            vput(e_im[s], k, sn);
+                            const int4 xv = sX[k * TH + tid];
+                            P[k] = (uint32_t)op.h[0] * (uint32_t)xv.x + (uint32_t)op.h[1] * (uint32_t)xv.y +
+                                   (uint32_t)op.h[2] * (uint32_t)xv.z + (uint32_t)op.h[3];
                         }
+#pragma unroll
+                        for (int k = 0; k < NA; k++) {
+                            const float4 xl = sXl[k * TH + tid];
+                            vput(lo, k, op.hf[0] * xl.x + op.hf[1] * xl.y + op.hf[2] * xl.z);
+                        }
+                        sincos_fixed_v<V>(P, lo, &e_im[s], &e_re[s]);
                     }
                 }
             } else {
@@ -552,9 +623,10 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
             const R2 g = sG[hl];
             V fs = anre, r[5];
             if constexpr (!TABLE) {
-                R rr[NA][6];
+                constexpr int NR = SAME ? 1 : NA;
+                R rr[NR][6];
 #pragma unroll
-                for (int k = 0; k < NA; k++) {
+                for (int k = 0; k < NR; k++) {
                     const R *rad = reinterpret_cast<const R *>(st + SL.tr + toff[k]) + 8 * hl;
                     if constexpr (IAM) {
                         rr[k][0] = rad[0];
@@ -571,13 +643,13 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                 }
                 V f0;
 #pragma unroll
-                for (int k = 0; k < NA; k++) vput(f0, k, rr[k][0]);
+                for (int k = 0; k < NA; k++) vput(f0, k, rr[k % NR][0]);
                 fs = vadd(fs, f0);
                 if constexpr (HC) {
 #pragma unroll
-                    for (int l = 0; l < 5; l++)
+                    for (int l = 0; l < NL; l++)
 #pragma unroll
-                        for (int k = 0; k < NA; k++) vput(r[l], k, rr[k][1 + l]);
+                        for (int k = 0; k < NA; k++) vput(r[l], k, rr[k % NR][1 + l]);
                 }
             }
             V Tiso = vdup<V>(R(1)), gre = vdup<V>(g.x), gim = vdup<V>(g.y);
@@ -749,7 +821,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                             if (slot_used<CS, PAT>(2, k)) E[k] = k == 0 ? vfma(r[2], A[2][k], E[k]) : vmul(r[2], A[2][k]);
                             if (slot_used<CS, PAT>(1, k)) O[k] = k == 0 ? vfma(r[1], A[1][k], O[k]) : vmul(r[1], A[1][k]);
                         }
-                        if (high_l) {
+                        if constexpr (HL) {
 #pragma unroll
                             for (int q = 9; q < 25; q++) {
                                 const int l = harmonic_l(q), k = pk_char<CS, PAT>(harmonic_class(q));
@@ -773,7 +845,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                             fr[s] = fi[s] = vdup<V>(R(0));
                             if constexpr (F64 && TABLE) {
                                 if (active[0]) {
-                                    const size_t a = (size_t)a_begin + slot;
+                                    const size_t a = (size_t)atom[0];
                                     const size_t col = a + (a >= (size_t)S.table_split ? S.table_shift : 0);
                                     const size_t ti = ((size_t)(h0 + hl) * S.table_stride + col) * NSC + op;
                                     if (S.table_d) {
@@ -848,24 +920,24 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                         V dr[7];
 #pragma unroll
                         for (int k = 0; k < NA; k++) {
-                            const R *rm = reinterpret_cast<const R *>(st + SL.trm + toff[k]) + 8 * hl;
+                            const R *rm = reinterpret_cast<const R *>(st + SL.trm + toff[SAME ? 0 : k]) + 8 * hl;
 #pragma unroll
                             for (int q = 0; q < 7; q++) vput(dr[q], k, rm[q]);
                         }
                         part[CH_PV] = vfma(dr[0], We[0], part[CH_PV]);
                         part[CH_KAPPA] = vfma(dr[1], We[0], part[CH_KAPPA]);
                         // kappa' and the populations: per (l, character) slot the weight r_l We (even l), -r_l Wo (odd l)
+                        V kp;  // the reflection's kappa' sum apart: one rounding into the running sum
 #pragma unroll
                         for (int l = 0; l < 5; l++) {
-                            if (l >= 3 && !high_l) continue;
+                            if (l >= NL) continue;
                             V QC[CS];
 #pragma unroll
                             for (int k = 0; k < CS; k++) {
                                 if (!slot_used<CS, PAT>(l, k)) continue;
                                 const V Wk = (l & 1) ? Wo[k] : We[k];
                                 const V t = vmul(A[l][k], Wk);
-                                part[CH_KAPPA_P] = (l & 1) ? vfnma(dr[2 + l], t, part[CH_KAPPA_P])
-                                                           : vfma(dr[2 + l], t, part[CH_KAPPA_P]);
+                                kp = l == 0 ? vmul(dr[2], t) : (l & 1) ? vfnma(dr[2 + l], t, kp) : vfma(dr[2 + l], t, kp);
                                 QC[k] = vmul(r[l], Wk);
                             }
 #pragma unroll
@@ -875,19 +947,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                                                            : vfma(Qk, cr[q], part[CH_PLM + q]);
                             }
                         }
-                        if (!high_l) {
-                            // populations of l = 3, 4 may exist with zero values (their derivatives do not vanish)
-#pragma unroll
-                            for (int l = 3; l < 5; l++) {
-#pragma unroll
-                                for (int q = l * l; q < (l + 1) * (l + 1); q++) {
-                                    const int k = pk_char<CS, PAT>(harmonic_class(q));
-                                    const V Qk = vmul(r[l], (l & 1) ? Wo[k] : We[k]);
-                                    part[CH_PLM + q] = (l & 1) ? vfnma(Qk, cr[q], part[CH_PLM + q])
-                                                               : vfma(Qk, cr[q], part[CH_PLM + q]);
-                                }
-                            }
-                        }
+                        part[CH_KAPPA_P] = vadd(part[CH_KAPPA_P], kp);
                     }
                 }
                 if constexpr (GRAD) {
@@ -929,20 +989,29 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
 #pragma unroll 1
             for (int g0 = seg0; g0 < seg0 + seg; g0 += 4) {
                 R Fv[8];
-                if constexpr (ROLL_J) {
+                // a group inside its lines runs as one straight stretch of code; one with a line start takes its
+                // reflections in a loop (with large bodies every group does)
+                bool straight = false;
+                if constexpr (!ROLL_J) {
+                    const int4 c4 = *reinterpret_cast<const int4 *>(sCont + g0);
+                    straight = (c4.x & c4.y & c4.z & c4.w) != 0 && !(g0 == seg0 && fresh);
+                }
+                if (straight) {
+                    if constexpr (!ROLL_J) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++) reflection(g0 + j, PkNo{}, Fv[2 * j], Fv[2 * j + 1]);
+                    }
+                } else {
 #pragma unroll
                     for (int q = 0; q < 8; q++) Fv[q] = R(0);
 #pragma unroll 1
                     for (int j = 0; j < 4; j++) {
                         R a, b;
-                        reflection(g0 + j, a, b);
+                        reflection(g0 + j, PkYes{}, a, b);
 #pragma unroll
                         for (int q = 0; q < 4; q++)
                             if (q == j) { Fv[2 * q] = a; Fv[2 * q + 1] = b; }
                     }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) reflection(g0 + j, Fv[2 * j], Fv[2 * j + 1]);
                 }
                 const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
                 R v4[4], v2[2];
@@ -966,10 +1035,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                 }
             }
         } else {
-            for (int i = seg0 + lane; i < seg0 + seg; i += 32) {
-                sF[warp * ht + i].x = R(0);
-                sF[warp * ht + i].y = R(0);
-            }
+            for (int i = seg0 + lane; i < seg0 + seg; i += 32) sF[warp * ht + i] = R2{R(0), R(0)};
         }
         if (GRAD && ((k_sub + 1) % fold == 0 || h0 + ht >= h_end)) {
 #pragma unroll
@@ -1005,7 +1071,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
 #pragma unroll
         for (int k = 0; k < NA; k++) {
             if (!active[k]) continue;
-            double *G = C.g_acc + ((size_t)a_begin + slot * NA + k) * kNch;
+            double *G = C.g_acc + (size_t)atom[k] * kNch;
             auto total = [&](int q) {
                 const int col = q * kTileAtoms + k * TH + tid;
                 const double t = (double)sTot[col] - (double)sCmp[col];
@@ -1020,16 +1086,76 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     }
 }
 
-// one structure, both ADP kinds in one launch: block (tile, reflection chunk)
-template <typename V, int MODEL, bool MP, int NSC, int CS, bool GRAD, bool INV, int PAT>
-__global__ void __launch_bounds__(pk_threads<V>())
+// a block's tile: the code of its ADP kind and of its angular sums (with or without l = 3, 4).  KIND 0, 1: the launch
+// holds tiles without, with anisotropic ADPs only
+template <typename V, int MODEL, bool MP, int NSC, int CS, bool GRAD, bool INV, int PAT, int KIND, bool ROLL>
+__device__ __forceinline__ void pk_tile(const DevStructure &S, const CallBuffers &C, const PkLaunch &L, int tile,
+                                        int chunk)
+{
+    const bool aniso = KIND == 1 || (KIND == 2 && tile >= L.T.n_plain);
+    if constexpr (MODEL == MODEL_HC) {
+        const int4 info = L.T.info[tile];
+        if ((MP ? info.w : info.z) >= 3) {
+            if (KIND != 0 && aniso) pk_body<V, MODEL, MP, KIND != 0, NSC, CS, GRAD, INV, PAT, ROLL, true>(S, C, L, tile, chunk);
+            else pk_body<V, MODEL, MP, KIND == 1, NSC, CS, GRAD, INV, PAT, ROLL, true>(S, C, L, tile, chunk);
+            return;
+        }
+    }
+    if (KIND != 0 && aniso) pk_body<V, MODEL, MP, KIND != 0, NSC, CS, GRAD, INV, PAT, ROLL, false>(S, C, L, tile, chunk);
+    else pk_body<V, MODEL, MP, KIND == 1, NSC, CS, GRAD, INV, PAT, ROLL, false>(S, C, L, tile, chunk);
+}
+
+// Blocks per SM that the register allocation aims at.  Two atoms per thread: six (168 registers, three warps per
+// scheduler), but the compiler's choice (about 220, two warps) where the cap would spill: HC derivatives with cosets of
+// four (5,000 isotropic atoms, P2_1 2_1 2_1: 1.48 ms without, 1.55 ms with the cap; 4,000 atoms, C2/c 1.11 and
+// 1.03 ms).  One atom, FP32 without the multipole adjoint: four (128 registers; 96 and 168 within 4% of it).
+template <typename V, int MODEL, bool MP, bool GRAD, int CS>
+__host__ __device__ constexpr int pk_min_blocks()
+{
+    if (VTraits<V>::NA == 2) return MODEL == MODEL_HC && GRAD && CS == 4 ? 1 : 6;
+    return sizeof(V) == 4 && !MP ? 4 : 1;
+}
+
+// one structure: block (reflection chunk, tile), so that blocks that run together share a tile's code and types.  KIND
+// 2: both ADP kinds in one launch (FP64, and FP32 grids of a few blocks per SM, where a second launch costs more than
+// it saves); 0, 1: one launch per kind (two kinds' code at once overflow the instruction caches)
+template <typename V, int MODEL, bool MP, int NSC, int CS, bool GRAD, bool INV, int PAT, int KIND>
+__global__ void __launch_bounds__(pk_threads<V>(), pk_min_blocks<V, MODEL, MP, GRAD, CS>())
 pk_kernel(const __grid_constant__ DevStructure S, const __grid_constant__ CallBuffers C,
           const __grid_constant__ PkLaunch L)
 {
-    if ((int)blockIdx.x < L.n_plain)
-        pk_body<V, MODEL, MP, false, NSC, CS, GRAD, INV, PAT>(S, C, L, blockIdx.x, blockIdx.y);
-    else
-        pk_body<V, MODEL, MP, true, NSC, CS, GRAD, INV, PAT>(S, C, L, blockIdx.x, blockIdx.y);
+    pk_tile<V, MODEL, MP, NSC, CS, GRAD, INV, PAT, KIND, KIND == 2>(
+        S, C, L, blockIdx.y + (KIND == 1 ? L.T.n_plain : 0), blockIdx.x);
+}
+
+// many structures of one kernel form in one launch (kernel-parameter space holds up to kBatchItems): the block's item
+// is the last with block_begin <= blockIdx.x
+struct PkBatchItem {
+    DevStructure S;
+    CallBuffers C;
+    PkLaunch L;
+    int n_tiles;
+};
+struct PkBatch {
+    int n;
+    int block_begin[kBatchItems + 1];
+    PkBatchItem item[kBatchItems];
+};
+
+template <typename V, int MODEL, int NSC, int CS, bool INV, int PAT>
+__global__ void __launch_bounds__(pk_threads<V>(), pk_min_blocks<V, MODEL, false, true, CS>())
+pk_batch_kernel(const __grid_constant__ PkBatch B)
+{
+    const int b = blockIdx.x;
+    int lo = 0, hi = B.n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (B.block_begin[mid] <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    const PkBatchItem &it = B.item[lo];
+    const int lb = b - B.block_begin[lo], n_chunks = (B.block_begin[lo + 1] - B.block_begin[lo]) / it.n_tiles;
+    pk_tile<V, MODEL, false, NSC, CS, true, INV, PAT, 2, true>(it.S, it.C, it.L, lb / n_chunks, lb % n_chunks);
 }
 
 }  // namespace dsf

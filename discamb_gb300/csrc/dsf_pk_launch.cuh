@@ -17,8 +17,10 @@ struct PkArgs {
     const DevStructure *S = nullptr;
     const CallBuffers *C = nullptr;
     const PkLaunch *L = nullptr;
+    const PkBatch *B = nullptr;  // a batched launch of `blocks` blocks instead of one structure's
     PkForm form;
-    int n_tiles = 0, n_chunks = 0;
+    bool split_kinds = false;    // one launch per ADP kind
+    int n_tiles = 0, n_chunks = 0, blocks = 0;
     size_t smem = 0;
     cudaStream_t st = nullptr;
 };
@@ -61,13 +63,39 @@ inline bool pk_generic_form(const PkForm &f, F &&go)
     return false;
 }
 
+template <typename K>
+cudaError_t launch_pk_tiles(K k, int threads, int n_tiles, const PkArgs &A)
+{
+    if (n_tiles <= 0) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A.smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(A.n_chunks, n_tiles), threads, A.smem, A.st>>>(*A.S, *A.C, *A.L);
+    return cudaGetLastError();
+}
+
 template <typename V, int MODEL, bool MP, bool GRAD, typename C>
 cudaError_t launch_pk(const PkArgs &A)
 {
-    auto k = pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT>;
+    constexpr int TH = pk_threads<V>();
+    if constexpr (sizeof(V) != sizeof(double) || VTraits<V>::NA == 2) {
+        if (A.split_kinds) {
+            const cudaError_t e = launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, 0>, TH,
+                                                  A.L->T.n_plain, A);
+            if (e != cudaSuccess) return e;
+            return launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, 1>, TH,
+                                   A.n_tiles - A.L->T.n_plain, A);
+        }
+    }
+    return launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, 2>, TH, A.n_tiles, A);
+}
+
+template <typename V, int MODEL, typename C>
+cudaError_t launch_pk_batch(const PkArgs &A)
+{
+    auto k = pk_batch_kernel<V, MODEL, C::N, C::CS, C::INV, C::PAT>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A.smem);
     if (e != cudaSuccess) return e;
-    k<<<dim3(A.n_tiles, A.n_chunks), pk_threads<V>(), A.smem, A.st>>>(*A.S, *A.C, *A.L);
+    k<<<A.blocks, pk_threads<V>(), A.smem, A.st>>>(*A.B);
     return cudaGetLastError();
 }
 
@@ -82,12 +110,31 @@ cudaError_t dispatch_pk(const PkArgs &A)
     return e;
 }
 
+template <typename V, int MODEL>
+cudaError_t dispatch_pk_batch(const PkArgs &A)
+{
+    cudaError_t e = cudaErrorInvalidValue;
+    auto go = [&](auto c) { e = launch_pk_batch<V, MODEL, decltype(c)>(A); };
+    if constexpr (MODEL == MODEL_HC) pk_hc_form(A.form, go);
+    else pk_generic_form(A.form, go);
+    return e;
+}
+
 // per-translation-unit entries
 cudaError_t launch_pk_f64_hc(const PkArgs &A);
 cudaError_t launch_pk_f64_hc_mp(const PkArgs &A);
 cudaError_t launch_pk_f64_hc_f(const PkArgs &A);
 cudaError_t launch_pk_f64_iam(const PkArgs &A);
 cudaError_t launch_pk_f64_table(const PkArgs &A);
+cudaError_t launch_pk_f32_hc(const PkArgs &A);
+cudaError_t launch_pk_f32_hc_f(const PkArgs &A);
+cudaError_t launch_pk_f32_iam(const PkArgs &A);
+cudaError_t launch_pk_f32_hc_mp(const PkArgs &A);
+cudaError_t launch_pk_f32_hc_batch(const PkArgs &A);
+cudaError_t launch_pk_f32_hc1(const PkArgs &A);
+cudaError_t launch_pk_f32_hc1_f(const PkArgs &A);
+cudaError_t launch_pk_f32_hc1_batch(const PkArgs &A);
+cudaError_t launch_pk_f32_iam_batch(const PkArgs &A);
 
 // record tables (dsf_prep_kernels.cu): kind 0: F2 slots (duplicated floats), 1: float slots, 2: double slots
 cudaError_t launch_pk_prep(const DevStructure &S, int n_hkl_pad, int cs, int kind, void *out, cudaStream_t st);

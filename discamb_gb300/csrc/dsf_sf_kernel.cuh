@@ -374,14 +374,13 @@ struct PhaseOps<double> {
 // step e^{2 pi i ((R^T e_l).x + e_l.t)} (the reference engine's line
 // recurrence, scattering_utilities::calculate_line_phase_factors,
 // src/Scattering/scattering_utilities.cpp:575-627); the exact phase is
-// re-anchored at every line start, at every sub-tile start and, in the FP32
-// form, every kAnchorF32 reflections so the FP32 rounding of the step cannot
-// build up.  With 16 (sub-tiles hold at most 16 reflections: an anchor at
-// every line and sub-tile start) the FP32 error against FP64 measured
-// 3.6e-7 (F) on the 5,000-atom P2_1 2_1 2_1 and 50,000-atom P4_3 2_1 2
-// structures and 2.2e-7 on a 256-crystal P2_1/c tabulated batch, against
-// 3.1-3.2e-7 and 1.6e-7 with 8, for 2.4-3.4% of the time.
-constexpr int kAnchorF32 = 16;
+// re-anchored at every line start, at every anchor_interval-th reflection of
+// a line (the cont flags of the reflection set say where) and at a block's
+// first reflection, so the FP32 rounding of the step cannot build up.  The
+// intervals keep the FP32 errors against FP64 where they were with anchors at
+// line starts and 8- or 16-reflection sub-tile starts (F 2.2-3.6e-7); 16
+// everywhere gave up to 11% more error for 1-3% less time.
+__host__ __device__ constexpr int anchor_interval(int n_sym) { return n_sym == 1 ? 6 : n_sym >= 8 ? 8 : 12; }
 
 // GRAD = false: structure factors only (the reference's calculateStructureFactors, which runs its engine with
 // every derivative switched off, HansenCoppensStructureFactorCalculator.cpp:305-326): the derivative sums are
@@ -414,7 +413,7 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
     constexpr bool XDIAG = CS > 0;
     constexpr int NSG = ADIAG ? 6 : (XDIAG ? 3 : 1);  // signed sums of u per coset
     constexpr bool WHT = PAT != 0 && CS == 4;
-    static_assert(PAT == 0 || CS == 4, "sign-group patterns: cosets of four");
+    static_assert(PAT == 0 || (CS == 4 && MODEL == MODEL_TABLE), "sign-group patterns: tabulated model, cosets of four");
     static_assert(CS == 0 || (NSC > 0 && NSC <= 8 && NSC % CS == 0), "coset form: compiled count <= 8");
     static_assert(GRAD || !MP, "the multipole adjoint needs the derivative pass");
     static_assert(!INV || (MODEL != MODEL_HC && NSC > 0 && NSC % 2 == 0), "inversion pairs: generic models, even count");
@@ -642,8 +641,7 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
             // reflection j of the group; its partial F goes to Fv[2j], Fv[2j + 1]
             auto reflection = [&](const int j) {
                 const int hl = g0 + j;
-                const bool anchor = !REC || sCont[hl] == 0 || hl == 0 ||
-                                    (F32 && (hl % kAnchorF32) == 0);
+                const bool anchor = !REC || sCont[hl] == 0 || (hl == 0 && k == 0);
                 if (active) {
                     const R2 g = sG[hl];
                     R fsre = anre, fsim = anim, r0 = 0, r1 = 0, r2 = 0, r3 = 0, r4 = 0;
@@ -729,25 +727,8 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
                     };
                     // coset form: radial-weighted class sums, even l (real part) and odd l (imaginary part)
                     R Ec[4] = {0, 0, 0, 0}, Oc[4] = {0, 0, 0, 0};  // classes 0 3 6 5 | 2 4 1 7
-                    // WHT: per position of the coset, the operations' f (HC), u and (multipole adjoint) g z
-                    R fwr[WHT ? 4 : 1], fwi[WHT ? 4 : 1], ur4[WHT ? 4 : 1], ui4[WHT ? 4 : 1];
-                    R wr4[WHT && MP ? 4 : 1], wi4[WHT && MP ? 4 : 1];
-                    // WHT (HC): each operation's f from the class sums gathered by character
-                    auto forward_wht = [&]() {
-                        if constexpr (WHT && DIAG) {
-                            constexpr int ec[4] = {0, 3, 6, 5}, oc[4] = {2, 4, 1, 7};
-                            R Ep[4] = {kZero<R>, kZero<R>, kZero<R>, kZero<R>}, t[4];
-                            R Op[4] = {kZero<R>, kZero<R>, kZero<R>, kZero<R>};
-#pragma unroll
-                            for (int q = 0; q < 4; q++) {
-                                Ep[wht_char(PAT, ec[q])] += Ec[q];
-                                Op[wht_char(PAT, oc[q])] += Oc[q];
-                            }
-                            wht4x2(Ep, Op, fwr, t);
-#pragma unroll
-                            for (int q = 0; q < 4; q++) fwi[q] = fsim + t[q];
-                        }
-                    };
+                    // WHT: per position of the coset, the operations' u
+                    R ur4[WHT ? 4 : 1], ui4[WHT ? 4 : 1];
                     // with the multipole adjoint: the same class sums weighted by the kappa'
                     // derivatives of the radial terms (De, Do), and the operations' signed
                     // adjoint weights per class (We: Re(g z) of the even classes, Wo: Im(g z) of
@@ -785,14 +766,6 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
                                         part[CH_ADP + q] -= m6r[q] * (gre * Wr[k] - gim * Wi[k]);
                                     }
                                 }
-                            }
-                            if constexpr (MP && DIAG) {
-                                R Vr[4], Vi[4];
-                                wht4x2(wr4, wi4, Vr, Vi);
-                                We[0] = Vr[0]; We[1] = Vr[wht_char(PAT, 3)]; We[2] = Vr[wht_char(PAT, 6)];
-                                We[3] = Vr[wht_char(PAT, 5)];
-                                Wo[0] = Vi[wht_char(PAT, 2)]; Wo[1] = Vi[wht_char(PAT, 4)]; Wo[2] = Vi[wht_char(PAT, 1)];
-                                Wo[3] = Vi[wht_char(PAT, 7)];
                             }
                         }
                     };
@@ -956,9 +929,6 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
                                 }
                                 fre = tv.x + anre; fim = tv.y + anim;
                             }
-                        } else if constexpr (DIAG && WHT) {
-                            fre = fwr[s & 3];
-                            fim = fwi[s & 3];
                         } else if constexpr (DIAG) {
                             // fsph rides in the class-0 sums (sign +1 for every operation)
                             if constexpr (F32) {
@@ -1031,13 +1001,8 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
                                 const auto sg = [&](int c) -> R {
                                     if constexpr (F32) return G.f[s][c]; else return G.d[s][c];
                                 };
-                                if constexpr (WHT) {
-                                    wr4[s & 3] = wre;
-                                    wi4[s & 3] = wim;
-                                } else {
                                 We[0] += wre; We[1] += sg(3) * wre; We[2] += sg(6) * wre; We[3] += sg(5) * wre;
                                 Wo[0] += sg(2) * wim; Wo[1] += sg(4) * wim; Wo[2] += sg(1) * wim; Wo[3] += sg(7) * wim;
-                                }
                             } else {
                                 const R *dr = sTrm + (size_t)(lt * ht + hl) * 8;
                                 Ere += zre; Eim += zim;
@@ -1070,7 +1035,6 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
                                     }
                                     class_sums(recs[s].y);
                                     mp_coset_begin(recs[s].y, sTrm + (size_t)(lt * ht + hl) * 8);
-                                    forward_wht();
                                     adp_coset_begin(recs[s]);
                                 }
                             }
@@ -1217,17 +1181,6 @@ template <typename R, int MODEL, bool MP, bool ANISO, int NSC, int CS = 0, bool 
           int PAT = 0>
 __global__ void __launch_bounds__(kTileAtoms)
 sf_grad_kernel3(DevStructure S, CallBuffers C, SfLaunch L, SignTable G)
-{
-    sf_grad_body<R, MODEL, MP, ANISO, NSC, CS, GRAD, INV, PAT>(S, C, L, G, blockIdx.x, blockIdx.y);
-}
-
-// the same with at least three blocks per SM: a register cap (168) for the FP32 multipole-adjoint kernels, which
-// the compiler otherwise gives about 220 registers (two blocks per SM); the autotuner times both and keeps the
-// faster (it trades a few spills for half again as many warps)
-template <typename R, int MODEL, bool MP, bool ANISO, int NSC, int CS = 0, bool GRAD = true, bool INV = false,
-          int PAT = 0>
-__global__ void __launch_bounds__(kTileAtoms, 3)
-sf_grad_kernel3_occ3(DevStructure S, CallBuffers C, SfLaunch L, SignTable G)
 {
     sf_grad_body<R, MODEL, MP, ANISO, NSC, CS, GRAD, INV, PAT>(S, C, L, G, blockIdx.x, blockIdx.y);
 }
