@@ -35,8 +35,7 @@
 
 namespace dsf {
 cudaError_t launch_rs_prep(const DevStructure &S, int n_hkl_pad, void *rs_f, void *rs_d, cudaStream_t st);
-cudaError_t launch_tr_prep(const DevStructure &S, int n_hkl_pad, void *tr_f, void *tr_d, void *trm_f, void *trm_d,
-                           bool mp, cudaStream_t st);
+cudaError_t launch_tr_prep(const DevStructure &S, int n_hkl_pad, bool fp64, void *tr, void *trm, cudaStream_t st);
 size_t rs_record_bytes(bool fp64);
 int tsc_expand(const char *path, int n_atoms, int n_hkl, const int *hkl, int ns, const int *rot,
                std::vector<float> &tab, std::string &err);
@@ -343,8 +342,7 @@ struct GradParams {
 // derivatives of atom a (engine order) in the crystal's conventions, original atom order
 __device__ __forceinline__ void grad_epilogue_one(int a, const GradParams &P, const double *g_acc, const int *perm,
                                                   const int *adpk, const double *w, const double *mult_w,
-                                                  const double *dmat, const int *plm_lmax, double *d_xyz,
-                                                  double *d_adp, double *d_occ, double *d_pval, double *d_plm,
+                                                  double *d_xyz, double *d_adp, double *d_occ, double *d_pval,
                                                   double *d_kappa, double *d_kappa_p)
 {
     const int o = perm[a];
@@ -377,32 +375,28 @@ __device__ __forceinline__ void grad_epilogue_one(int a, const GradParams &P, co
         if (d_pval) d_pval[o] = wa * G[CH_PV];
         if (d_kappa) d_kappa[o] = wa * G[CH_KAPPA];
         if (d_kappa_p) d_kappa_p[o] = wa * G[CH_KAPPA_P];
-        if (d_plm) {
-            const double *D = dmat + (size_t)a * 165;
-            int off = 0;
-            for (int l = 0; l <= 4; l++) {
-                const int n = 2 * l + 1;
-                for (int i = 0; i < n; i++) {
-                    double s = 0;
-                    for (int j = 0; j < n; j++) s += D[off + i * n + j] * G[CH_PLM + l * l + j];
-                    d_plm[25 * o + l * l + i] = l <= plm_lmax[a] ? wa * s : 0.0;
-                }
-                off += n * n;
-            }
-        }
     }
 }
 
+// derivative by population q of atom a (a thread each: 25 threads per atom)
+__device__ __forceinline__ void plm_epilogue_one(int a, int q, const double *g_acc, const int *perm, const double *w,
+                                                 const double *dmat, const int *plm_lmax, double *d_plm)
+{
+    const int l = q < 1 ? 0 : q < 4 ? 1 : q < 9 ? 2 : q < 16 ? 3 : 4, n = 2 * l + 1;
+    const double *D = dmat + (size_t)a * 165 + l * (2 * l - 1) * (2 * l + 1) / 3 + (q - l * l) * n;
+    const double *G = g_acc + (size_t)a * kNch + CH_PLM + l * l;
+    double s = 0;
+    for (int j = 0; j < n; j++) s += D[j] * G[j];
+    d_plm[25 * (size_t)perm[a] + q] = l <= plm_lmax[a] ? w[a] * s : 0.0;
+}
+
 __global__ void grad_epilogue_kernel(GradParams P, const double *g_acc, const int *perm, const int *adpk,
-                                     const double *w, const double *mult_w, const double *dmat,
-                                     const int *plm_lmax, double *d_xyz,
-                                     double *d_adp, double *d_occ, double *d_pval, double *d_plm, double *d_kappa,
-                                     double *d_kappa_p)
+                                     const double *w, const double *mult_w, double *d_xyz, double *d_adp,
+                                     double *d_occ)
 {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a < P.n_atoms)
-        grad_epilogue_one(a, P, g_acc, perm, adpk, w, mult_w, dmat, plm_lmax, d_xyz, d_adp, d_occ, d_pval, d_plm,
-                          d_kappa, d_kappa_p);
+        grad_epilogue_one(a, P, g_acc, perm, adpk, w, mult_w, d_xyz, d_adp, d_occ, nullptr, nullptr, nullptr);
 }
 
 // a single structure's call in two small launches around the structure-factor kernels: before them the adjoint
@@ -428,8 +422,9 @@ __global__ void call_post_kernel(int n_hkl, const double2 *facc, const double *m
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_hkl) f_epilogue_one(i, facc, mult, cinv, centro, f_out, hperm);
     if (grad && i < P.n_atoms)
-        grad_epilogue_one(i, P, g_acc, perm, adpk, w, mult_w, dmat, plm_lmax, d_xyz, d_adp, d_occ, d_pval, d_plm,
-                          d_kappa, d_kappa_p);
+        grad_epilogue_one(i, P, g_acc, perm, adpk, w, mult_w, d_xyz, d_adp, d_occ, d_pval, d_kappa, d_kappa_p);
+    if (grad && P.want_mp && d_plm && i < 25 * P.n_atoms)
+        plm_epilogue_one(i / 25, i % 25, g_acc, perm, w, dmat, plm_lmax, d_plm);
 }
 
 // multipole-parameter derivatives summed over the atoms of each type (atoms of
@@ -504,9 +499,11 @@ __global__ void batch_post_kernel(const __grid_constant__ PrePostBatch B)
         f_epilogue_one(i, it.facc, it.mult, it.cinv, it.centro, it.f_out, it.hperm);
     if (!it.want_grad) return;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < it.n_atoms; a += stride)
-        grad_epilogue_one(a, it.P, it.gacc, it.perm, it.adpk, it.w, it.mult_w, it.dmat, it.plm_lmax, it.out.d_xyz,
-                          it.out.d_adp, it.out.d_occ, it.out.d_pval, it.out.d_plm, it.out.d_kappa,
-                          it.out.d_kappa_prime);
+        grad_epilogue_one(a, it.P, it.gacc, it.perm, it.adpk, it.w, it.mult_w, it.out.d_xyz, it.out.d_adp,
+                          it.out.d_occ, it.out.d_pval, it.out.d_kappa, it.out.d_kappa_prime);
+    if (!it.P.want_mp || !it.out.d_plm) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 25 * it.n_atoms; i += stride)
+        plm_epilogue_one(i / 25, i % 25, it.gacc, it.perm, it.w, it.dmat, it.plm_lmax, it.out.d_plm);
 }
 
 struct AtomParams {
@@ -1232,19 +1229,15 @@ int ensure_tables(dsf_structure *s, bool fp64, bool mp)
         DSF_CUDA(launch_rs_prep(s->dev, s->n_hkl_pad, fp64 ? nullptr : rs.p, fp64 ? rs.p : nullptr, e->setup));
         s->rs_ok[p] = true;
     }
-    if (!s->tr_ok[p]) {
-        DevBuf &tr = fp64 ? s->d_tr_d : s->d_tr_f;
-        DSF_CUDA(tr.alloc(esz * row));
-        DSF_CUDA(launch_tr_prep(s->dev, s->n_hkl_pad, fp64 ? nullptr : tr.p, fp64 ? tr.p : nullptr, nullptr,
-                                nullptr, false, e->setup));
-        s->tr_ok[p] = true;
-    }
-    if (mp && !s->trm_ok[p]) {
-        DevBuf &trm = fp64 ? s->d_trm_d : s->d_trm_f;
-        DSF_CUDA(trm.alloc(esz * row));
-        DSF_CUDA(launch_tr_prep(s->dev, s->n_hkl_pad, nullptr, nullptr, fp64 ? nullptr : trm.p,
-                                fp64 ? trm.p : nullptr, true, e->setup));
-        s->trm_ok[p] = true;
+    DevBuf &tr = fp64 ? s->d_tr_d : s->d_tr_f, &trm = fp64 ? s->d_trm_d : s->d_trm_f;
+    const bool need_tr = !s->tr_ok[p], need_trm = mp && !s->trm_ok[p];
+    if (need_tr || need_trm) {
+        if (need_tr) DSF_CUDA(tr.alloc(esz * row));
+        if (need_trm) DSF_CUDA(trm.alloc(esz * row));
+        DSF_CUDA(launch_tr_prep(s->dev, s->n_hkl_pad, fp64, need_tr ? tr.p : nullptr, need_trm ? trm.p : nullptr,
+                                e->setup));
+        if (need_tr) s->tr_ok[p] = true;
+        if (need_trm) s->trm_ok[p] = true;
     }
     // the calls that read the tables may run on another stream
     if (built) DSF_CUDA(cudaStreamSynchronize(e->setup));
@@ -1445,9 +1438,8 @@ cudaError_t launch_grad_epilogue(int n_atoms, int xyz_conv, const double *Minv, 
     P.want_adp = (flags & DSF_D_ADP) != 0;
     P.want_occ = (flags & DSF_D_OCC) != 0;
     P.want_mp = 0;
-    grad_epilogue_kernel<<<(n_atoms + 127) / 128, 128, 0, st>>>(P, g_acc, perm, adpk, w, mult_w, nullptr, nullptr,
-                                                                 out->d_xyz, out->d_adp, out->d_occ, nullptr, nullptr,
-                                                                 nullptr, nullptr);
+    grad_epilogue_kernel<<<(n_atoms + 127) / 128, 128, 0, st>>>(P, g_acc, perm, adpk, w, mult_w, out->d_xyz, out->d_adp,
+                                                                out->d_occ);
     return cudaGetLastError();
 }
 }  // namespace dsf
@@ -1928,14 +1920,15 @@ int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl)
         s->hperm.resize(n_hkl);
         for (int i = 0; i < n_hkl; i++) s->hperm[i] = key[i].second;
     }
-    // cont: 1 where a reflection takes its phases from the one before; 0 at line starts and, so that the recurrence's
-    // rounding cannot build up, at every anchor_interval-th reflection of a line (there the phase is exact again)
-    const int anchor = anchor_interval(s->n_sym);
+    // cont: whether a reflection takes its phases from the one before (bit 0: FP32, bit 1: FP64); not at line starts
+    // and, so that the recurrence's rounding cannot build up, at every anchor_interval-th reflection of a line (there
+    // the phase is exact again)
+    const int anchor = anchor_interval(s->n_sym, false), anchor64 = anchor_interval(s->n_sym, true);
     std::vector<int> cont(n_pad, 0);
     for (int i = 1, run = 0; i < n_hkl; i++) {
         const int *p = hkl + 3 * s->hperm[i - 1], *q = hkl + 3 * s->hperm[i];
         run = (p[0] == q[0] && p[1] == q[1] && q[2] == p[2] + 1) ? run + 1 : 0;
-        cont[i] = run % anchor != 0;
+        cont[i] = (run % anchor != 0 ? 1 : 0) | (run % anchor64 != 0 ? 2 : 0);
     }
     std::vector<int4> h4(n_pad, make_int4(0, 0, 0, 0));
     std::vector<double> h2(n_pad, 0.0), mult(n_pad, 0.0), cinv(2 * (size_t)n_pad, 0.0);
@@ -2054,8 +2047,8 @@ int dsf_structure_update_types(dsf_structure *s, const double *plm, const double
     int rc;
     if ((rc = upload_types(s))) return rc;
     if (plm && (rc = compute_global_plm(s))) return rc;
+    // the radial tables are stale: a call builds the ones of its precision (and not the other's)
     for (int p = 0; p < 2; p++) s->tr_ok[p] = s->trm_ok[p] = false;
-    if ((rc = ensure_tables(s, false, false))) return rc;
     refresh_dev(s);
     DSF_CUDA(cudaStreamSynchronize(e->setup));
     return DSF_OK;
@@ -2246,7 +2239,7 @@ static int call_post(dsf_structure *s, int flags, const dsf_outputs *out, cudaSt
     P.want_adp = (flags & DSF_D_ADP) != 0;
     P.want_occ = (flags & DSF_D_OCC) != 0;
     P.want_mp = mp;
-    const int m = grad ? std::max(n_hkl, n) : n_hkl;
+    const int m = grad ? std::max(n_hkl, mp ? 25 * n : n) : n_hkl;
     call_post_kernel<<<(m + 127) / 128, 128, 0, st>>>(
         n_hkl, s->d_facc.as<double2>(), s->d_hmult.as<double>(), s->d_cinv.as<double2>(), s->centro_mode, out->f,
         s->d_hperm.as<int>(), grad ? 1 : 0, P, s->d_gacc.as<double>(), s->d_perm.as<int>(),
@@ -2262,10 +2255,10 @@ static int call_post(dsf_structure *s, int flags, const dsf_outputs *out, cudaSt
 // blocks of unequal tiles even out across the SMs, but at least 256 reflections (16 sub-tiles) per block so the
 // per-block set-up (atom loads, the final derivative commits) stays small -- unless that leaves fewer than four
 // blocks per SM (small structures)
-static int chunk_count(const dsf_engine *e, int ntk, int n_hkl, int blocks_per_sm = 75)
+static int chunk_count(const dsf_engine *e, int ntk, int n_hkl, int blocks_per_sm = 75, int least = 4)
 {
     const int sm = std::max(1, e->n_sm), t = std::max(1, ntk);
-    return std::max(1, std::max(std::min(sm * blocks_per_sm / t, n_hkl / 256), sm * 4 / t));
+    return std::max(1, std::max(std::min(sm * blocks_per_sm / t, n_hkl / 256), sm * least / t));
 }
 
 // ---------------------------------------------------------------------------
@@ -2376,7 +2369,8 @@ static int launch_pk_structure(dsf_structure *s, int kind, bool mp, bool grad, i
     PkLaunch L;
     PkArgs A;
     const int n_tiles = pk_map(s, kind).n_tiles;
-    const int n_chunks0 = chunk_count(e, n_tiles, s->n_hkl, bps);
+    // FP64: at least two blocks per SM (what is resident), so that a small structure's blocks pay their set-up once
+    const int n_chunks0 = chunk_count(e, n_tiles, s->n_hkl, bps, kind == 2 ? 2 : 4);
     const int want = std::max(1, (s->n_hkl + n_chunks0 - 1) / n_chunks0);
     const bool hc = s->model == MODEL_HC;
     mp = mp && hc;

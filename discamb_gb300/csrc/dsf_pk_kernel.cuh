@@ -375,7 +375,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw);
     const PkStage<V> SL(ht, REC, L.T.max_types, MP, TABLE);
     unsigned char *stage0 = smem_raw + 64;
-    R2 *sF = reinterpret_cast<R2 *>(stage0 + 2 * SL.bytes);  // [WARPS][ht]
+    R2 *sF = reinterpret_cast<R2 *>(stage0 + 2 * SL.bytes);  // [warps of a part][ht]
     R *sTot = reinterpret_cast<R *>(sF + WARPS * ht);        // [NT][kTileAtoms], Kahan total and compensation
     R *sCmp = sTot + (GRAD ? NT * kTileAtoms : 0);
     unsigned char *sp = reinterpret_cast<unsigned char *>(sCmp + (GRAD ? NT * kTileAtoms : 0));
@@ -390,11 +390,13 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     if constexpr (!F64) sp += 32 * kTileAtoms;
     int *sTypes = reinterpret_cast<int *>(sp);
 
-    // Small tiles: the block's threads in `split` parts of TH / split atom slots (whole warps), each part taking its
-    // own stretch of every sub-tile, so a tile of few atoms still uses every warp (and every FP64 sub-unit)
+    // Small tiles: the block's threads in `split` parts of TH / split atom slots (at least eight lanes), each part
+    // taking its own stretch of every sub-tile, so a tile of few atoms still uses every warp, every FP64 sub-unit and
+    // most lanes (an FP64 instruction costs the same however many lanes are in use)
     int slots = TH;
-    while (slots > 32 && slots / 2 * NA >= n_at && ht * slots / TH > 4) slots >>= 1;
+    while (slots > 8 && slots / 2 * NA >= n_at && ht * slots / 2 >= TH) slots >>= 1;
     const int split = TH / slots, part_id = tid / slots, slot = tid - part_id * slots;
+    const int width = min(slots, 32), wrow = slot / 32;  // lanes of a part inside a warp, the warp's row of sF
     const int seg = ht / split, seg0 = part_id * seg;  // this thread's reflections of a sub-tile: [seg0, seg0 + seg)
 
     for (int i = tid; i < nT; i += TH) sTypes[i] = L.T.types[tile * kMaxTileTypes + i];
@@ -577,7 +579,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
             const PkOp *ops = reinterpret_cast<const PkOp *>(rec);
             const V *cos_rec = reinterpret_cast<const V *>(rec + sizeof(PkOp) * NSC);
             // ---- phases: exact at line and stretch starts, one complex multiplication per operation in between
-            if (decltype(may_anchor)::value && (sCont[hl] == 0 || (hl == seg0 && fresh))) {
+            if (decltype(may_anchor)::value && ((sCont[hl] & (F64 ? 2 : 1)) == 0 || (hl == seg0 && fresh))) {
 #pragma unroll
                 for (int s = 0; s < NZ; s++) {
                     const PkOp op = ops[s];
@@ -988,13 +990,16 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
         if (warp_any) {
 #pragma unroll 1
             for (int g0 = seg0; g0 < seg0 + seg; g0 += 4) {
+                const int ng = min(4, seg);
                 R Fv[8];
                 // a group inside its lines runs as one straight stretch of code; one with a line start takes its
                 // reflections in a loop (with large bodies every group does)
                 bool straight = false;
                 if constexpr (!ROLL_J) {
+                    if (ng == 4) {
                     const int4 c4 = *reinterpret_cast<const int4 *>(sCont + g0);
-                    straight = (c4.x & c4.y & c4.z & c4.w) != 0 && !(g0 == seg0 && fresh);
+                    straight = (c4.x & c4.y & c4.z & c4.w & (F64 ? 2 : 1)) != 0 && !(g0 == seg0 && fresh);
+                    }
                 }
                 if (straight) {
                     if constexpr (!ROLL_J) {
@@ -1005,7 +1010,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
 #pragma unroll
                     for (int q = 0; q < 8; q++) Fv[q] = R(0);
 #pragma unroll 1
-                    for (int j = 0; j < 4; j++) {
+                    for (int j = 0; j < ng; j++) {
                         R a, b;
                         reflection(g0 + j, PkYes{}, a, b);
 #pragma unroll
@@ -1013,29 +1018,30 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                             if (q == j) { Fv[2 * q] = a; Fv[2 * q + 1] = b; }
                     }
                 }
-                const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+                // eight values over the part's lanes: halves, quarters, eighths of them, then their sums
+                const int o4 = width >> 1, o3 = width >> 2, o2 = width >> 3;
+                const bool b4 = lane & o4, b3 = lane & o3, b2 = lane & o2;
                 R v4[4], v2[2];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const R keep = b4 ? Fv[q + 4] : Fv[q], send = b4 ? Fv[q] : Fv[q + 4];
-                    v4[q] = keep + shfl_xor<R>(send, 16);
+                    v4[q] = keep + shfl_xor<R>(send, o4);
                 }
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
                     const R keep = b3 ? v4[q + 2] : v4[q], send = b3 ? v4[q] : v4[q + 2];
-                    v2[q] = keep + shfl_xor<R>(send, 8);
+                    v2[q] = keep + shfl_xor<R>(send, o3);
                 }
-                R v1 = (b2 ? v2[1] : v2[0]) + shfl_xor<R>(b2 ? v2[0] : v2[1], 4);
-                v1 += shfl_xor<R>(v1, 2);
-                v1 += shfl_xor<R>(v1, 1);
-                if ((lane & 3) == 0) {
-                    const int idx = lane >> 2;
-                    R *dst = reinterpret_cast<R *>(&sF[warp * ht + g0 + (idx >> 1)]);
+                R v1 = (b2 ? v2[1] : v2[0]) + shfl_xor<R>(b2 ? v2[0] : v2[1], o2);
+                for (int o = o2 >> 1; o > 0; o >>= 1) v1 += shfl_xor<R>(v1, o);
+                const int idx = (b4 ? 4 : 0) + (b3 ? 2 : 0) + (b2 ? 1 : 0);
+                if ((lane & (o2 - 1)) == 0 && (idx >> 1) < ng) {
+                    R *dst = reinterpret_cast<R *>(&sF[wrow * ht + g0 + (idx >> 1)]);
                     dst[idx & 1] = v1;
                 }
             }
         } else {
-            for (int i = seg0 + lane; i < seg0 + seg; i += 32) sF[warp * ht + i] = R2{R(0), R(0)};
+            for (int i = seg0 + lane % width; i < seg0 + seg; i += width) sF[wrow * ht + i] = R2{R(0), R(0)};
         }
         if (GRAD && ((k_sub + 1) % fold == 0 || h0 + ht >= h_end)) {
 #pragma unroll
@@ -1053,10 +1059,8 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
         }
         __syncthreads();
         for (int i = tid; i < ht; i += TH) {
-            // the warps of the part that took reflection i
-            const int w0 = i / seg * (slots / 32), w1 = w0 + slots / 32;
-            R sre = 0, sim = 0;
-            for (int wp = w0; wp < w1; wp++) {
+            R sre = 0, sim = 0;  // over the warps of the part that took reflection i
+            for (int wp = 0; wp < max(1, slots / 32); wp++) {
                 const R2 v = sF[wp * ht + i];
                 sre += v.x;
                 sim += v.y;

@@ -173,7 +173,7 @@ struct SfLaunch {
     const void *rs;        // RsRec<R> [n_hkl_pad][n_sym]
     const void *tr;        // R [n_types][n_hkl_pad][8]
     const void *trm;       // R [n_types][n_hkl_pad][8] (multipole adjoint)
-    const int *cont;       // [n_hkl_pad] 1: reflection = previous one + (0,0,1) (reflections in line order)
+    const int *cont;       // [n_hkl_pad] bit 0 (FP32), 1 (FP64): the phases follow from the reflection before, + (0,0,1)
     const int *tile_lmax;  // [n_tiles] highest l of the angular sums of the tile's atoms
     int *error;            // set to 1 on a timed-out wait
     int stall_first;       // test hook (dsf_debug_stall_next_call): the first sub-tile's copies are not issued, so
@@ -379,8 +379,11 @@ struct PhaseOps<double> {
 // first reflection, so the FP32 rounding of the step cannot build up.  The
 // intervals keep the FP32 errors against FP64 where they were with anchors at
 // line starts and 8- or 16-reflection sub-tile starts (F 2.2-3.6e-7); 16
-// everywhere gave up to 11% more error for 1-3% less time.
-__host__ __device__ constexpr int anchor_interval(int n_sym) { return n_sym == 1 ? 6 : n_sym >= 8 ? 8 : 12; }
+// everywhere gave up to 11% more error for 1-3% less time.  FP64: 16 (its error is that of the sums).
+__host__ __device__ constexpr int anchor_interval(int n_sym, bool fp64)
+{
+    return fp64 ? 16 : n_sym == 1 ? 6 : n_sym >= 8 ? 8 : 12;
+}
 
 // GRAD = false: structure factors only (the reference's calculateStructureFactors, which runs its engine with
 // every derivative switched off, HansenCoppensStructureFactorCalculator.cpp:305-326): the derivative sums are
@@ -641,7 +644,7 @@ __device__ __forceinline__ void sf_grad_body(const DevStructure &S, const CallBu
             // reflection j of the group; its partial F goes to Fv[2j], Fv[2j + 1]
             auto reflection = [&](const int j) {
                 const int hl = g0 + j;
-                const bool anchor = !REC || sCont[hl] == 0 || (hl == 0 && k == 0);
+                const bool anchor = !REC || (sCont[hl] & (F32 ? 1 : 2)) == 0 || (hl == 0 && k == 0);
                 if (active) {
                     const R2 g = sG[hl];
                     R fsre = anre, fsim = anim, r0 = 0, r1 = 0, r2 = 0, r3 = 0, r4 = 0;
