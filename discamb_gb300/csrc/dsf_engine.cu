@@ -768,20 +768,24 @@ PkForm pk_form_of(const dsf_structure *s)
     PkForm f;
     f.n_sym = n;
     f.inv = !hc && s->inv_pairs != 0;
+    f.cen = hc && s->centro_mode == 1;
     for (const int pat : {kPatD2, kPatC2hB})
         if (cosets(4, pat & 7, pat >> 3)) {
             f.cs = 4;
             f.pat = pat;
+            f.cen = f.cen && n == 4;
             return f;
         }
     for (const int a : {kPat2Y, kPat2Z, kPatInv})
         if (cosets(2, a, 0)) {
             f.cs = 2;
             f.pat = a;
+            f.cen = f.cen && n == 2;
             return f;
         }
     f.cs = 1;
     f.inv = false;
+    f.cen = f.cen && n == 1;
     return f;
 }
 
@@ -832,7 +836,6 @@ int sym_from_desc(dsf_engine *e, dsf_structure *s, const dsf_symmetry *sym)
         }
         s->inv_pairs = pairs ? 1 : 0;
     }
-    s->pk = pk_form_of(s);
     s->centro_mode = 0;
     if (sym->centrosymmetric) {
         bool origin = true;
@@ -847,6 +850,7 @@ int sym_from_desc(dsf_engine *e, dsf_structure *s, const dsf_symmetry *sym)
         }
         s->centro_mode = origin ? 1 : 2;
     }
+    s->pk = pk_form_of(s);
     s->centering = sym->centering ? sym->centering : 'P';
     s->obverse = sym->obverse;
     s->n_total = sym->n_symops_total > 0 ? sym->n_symops_total : s->n_sym;
@@ -2732,7 +2736,7 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
             PkGroup *g = nullptr;
             for (auto &x : pk_groups)
                 if (x.model == s->model && x.kind == pk && x.form.n_sym == s->pk.n_sym && x.form.cs == s->pk.cs &&
-                    x.form.pat == s->pk.pat && x.form.inv == s->pk.inv)
+                    x.form.pat == s->pk.pat && x.form.inv == s->pk.inv && x.form.cen == s->pk.cen)
                     g = &x;
             if (!g) {
                 pk_groups.emplace_back();

@@ -7,10 +7,11 @@ namespace dsf {
 
 // the symmetry form of a launch: n_sym operations in cosets of cs that form the sign group pat (cs = 4: kPatD2,
 // kPatC2hB; cs = 2: the mask of the axes that the second operation flips); inv: the second half of the operations
-// are the images of the first half under an inversion at the origin
+// are the images of the first half under an inversion at the origin; cen: the engine takes an inversion at the origin
+// beside them (HC; the common groups: -1, 2/m, mmm -- others run the general kernels, which are right for them too)
 struct PkForm {
     int n_sym = 0, cs = 0, pat = 0;
-    bool inv = false;
+    bool inv = false, cen = false;
 };
 
 struct PkArgs {
@@ -30,25 +31,32 @@ constexpr int kPat2Y = 5, kPat2Z = 3, kPatInv = 7;  // cs = 2: a two-fold axis a
 // runs f with the compile-time form that equals `f0`, one of the compiled ones of the model; false when none does.
 //   HC (operations without the inversion): P1 and P-1; P2_1, P2_1/c, C2/c; P4_1; 222; 422
 //   other models (all operations modulo centring): 1; 2; -1; 222; 2/m; mmm; any eight
-template <int N_, int CS_, int PAT_, bool INV_ = false>
+template <int N_, int CS_, int PAT_, bool INV_ = false, bool CEN_ = false>
 struct PkC {
     static constexpr int N = N_, CS = CS_, PAT = PAT_;
-    static constexpr bool INV = INV_;
+    static constexpr bool INV = INV_, CEN = CEN_;
 };
 template <typename C>
 inline bool pk_is(const PkForm &f)
 {
-    return f.n_sym == C::N && f.cs == C::CS && (C::CS == 1 || f.pat == C::PAT) && f.inv == C::INV;
+    return f.n_sym == C::N && f.cs == C::CS && (C::CS == 1 || f.pat == C::PAT) && f.inv == C::INV && f.cen == C::CEN;
+}
+template <bool CEN, typename F>
+inline bool pk_hc_form_of(const PkForm &f, F &&go)
+{
+    if (pk_is<PkC<1, 1, 0, false, CEN> >(f)) return go(PkC<1, 1, 0, false, CEN>{}), true;
+    if (pk_is<PkC<2, 2, kPat2Y, false, CEN> >(f)) return go(PkC<2, 2, kPat2Y, false, CEN>{}), true;
+    if (pk_is<PkC<4, 4, kPatD2, false, CEN> >(f)) return go(PkC<4, 4, kPatD2, false, CEN>{}), true;
+    if constexpr (!CEN) {
+        if (pk_is<PkC<4, 2, kPat2Z> >(f)) return go(PkC<4, 2, kPat2Z>{}), true;
+        if (pk_is<PkC<8, 4, kPatD2> >(f)) return go(PkC<8, 4, kPatD2>{}), true;
+    }
+    return false;
 }
 template <typename F>
 inline bool pk_hc_form(const PkForm &f, F &&go)
 {
-    if (pk_is<PkC<1, 1, 0> >(f)) return go(PkC<1, 1, 0>{}), true;
-    if (pk_is<PkC<2, 2, kPat2Y> >(f)) return go(PkC<2, 2, kPat2Y>{}), true;
-    if (pk_is<PkC<4, 2, kPat2Z> >(f)) return go(PkC<4, 2, kPat2Z>{}), true;
-    if (pk_is<PkC<4, 4, kPatD2> >(f)) return go(PkC<4, 4, kPatD2>{}), true;
-    if (pk_is<PkC<8, 4, kPatD2> >(f)) return go(PkC<8, 4, kPatD2>{}), true;
-    return false;
+    return f.cen ? pk_hc_form_of<true>(f, go) : pk_hc_form_of<false>(f, go);
 }
 template <typename F>
 inline bool pk_generic_form(const PkForm &f, F &&go)
@@ -79,20 +87,20 @@ cudaError_t launch_pk(const PkArgs &A)
     constexpr int TH = pk_threads<V>();
     if constexpr (sizeof(V) != sizeof(double) || VTraits<V>::NA == 2) {
         if (A.split_kinds) {
-            const cudaError_t e = launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, 0>, TH,
+            const cudaError_t e = launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, C::CEN, 0>, TH,
                                                   A.L->T.n_plain, A);
             if (e != cudaSuccess) return e;
-            return launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, 1>, TH,
+            return launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, C::CEN, 1>, TH,
                                    A.n_tiles - A.L->T.n_plain, A);
         }
     }
-    return launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, 2>, TH, A.n_tiles, A);
+    return launch_pk_tiles(pk_kernel<V, MODEL, MP, C::N, C::CS, GRAD, C::INV, C::PAT, C::CEN, 2>, TH, A.n_tiles, A);
 }
 
 template <typename V, int MODEL, typename C>
 cudaError_t launch_pk_batch(const PkArgs &A)
 {
-    auto k = pk_batch_kernel<V, MODEL, C::N, C::CS, C::INV, C::PAT>;
+    auto k = pk_batch_kernel<V, MODEL, C::N, C::CS, C::INV, C::PAT, C::CEN>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A.smem);
     if (e != cudaSuccess) return e;
     k<<<A.blocks, pk_threads<V>(), A.smem, A.st>>>(*A.B);
