@@ -323,6 +323,14 @@ struct PkTiles {
     int max_types;
 };
 
+template <typename R>
+struct PkEight {
+    R v[8];
+};
+template <int N>
+struct PkInt {
+    static constexpr int value = N;
+};
 struct PkYes {
     static constexpr bool value = true;
 };
@@ -994,12 +1002,52 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
             if constexpr (CEN) fi_out = R(0);
             else fi_out = vsum(vmul(wT, Uim));
         };
+        // a group's partial F over the lanes of the part, into sF
+        auto reduce = [&](const PkEight<R> &F8, auto w32, const int g0, const int ng) {
+            const R (&Fv)[8] = F8.v;
+            const int wd = decltype(w32)::value ? decltype(w32)::value : width;
+            const int o4 = wd >> 1, o3 = wd >> 2, o2 = wd >> 3;
+            const bool b4 = lane & o4, b3 = lane & o3, b2 = lane & o2;
+            if constexpr (CEN) {
+                // four real values over the part's lanes: halves, quarters of them, then their sums
+                R v2[2];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const R keep = b4 ? Fv[2 * q + 4] : Fv[2 * q], send = b4 ? Fv[2 * q] : Fv[2 * q + 4];
+                    v2[q] = keep + shfl_xor<R>(send, o4);
+                }
+                R v1 = (b3 ? v2[1] : v2[0]) + shfl_xor<R>(b3 ? v2[0] : v2[1], o3);
+                for (int o = o2; o > 0; o >>= 1) v1 += shfl_xor<R>(v1, o);
+                const int idx = (b4 ? 2 : 0) + (b3 ? 1 : 0);
+                if ((lane & (o3 - 1)) == 0 && idx < ng) sF[wrow * ht + g0 + idx] = R2{v1, R(0)};
+                return;
+            }
+            // eight values over the part's lanes: halves, quarters, eighths of them, then their sums
+            R v4[4], v2[2];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const R keep = b4 ? Fv[q + 4] : Fv[q], send = b4 ? Fv[q] : Fv[q + 4];
+                v4[q] = keep + shfl_xor<R>(send, o4);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const R keep = b3 ? v4[q + 2] : v4[q], send = b3 ? v4[q] : v4[q + 2];
+                v2[q] = keep + shfl_xor<R>(send, o3);
+            }
+            R v1 = (b2 ? v2[1] : v2[0]) + shfl_xor<R>(b2 ? v2[0] : v2[1], o2);
+            for (int o = o2 >> 1; o > 0; o >>= 1) v1 += shfl_xor<R>(v1, o);
+            const int idx = (b4 ? 4 : 0) + (b3 ? 2 : 0) + (b2 ? 1 : 0);
+            if ((lane & (o2 - 1)) == 0 && (idx >> 1) < ng) {
+                R *dst = reinterpret_cast<R *>(&sF[wrow * ht + g0 + (idx >> 1)]);
+                dst[idx & 1] = v1;
+            }
+        };
         // groups of four reflections: their eight sums over the warp by one butterfly reduce-scatter
         if (warp_any) {
 #pragma unroll 1
             for (int g0 = seg0; g0 < seg0 + seg; g0 += 4) {
                 const int ng = min(4, seg);
-                R Fv[8];
+                PkEight<R> Fv;
                 // a group inside its lines runs as one straight stretch of code; one with a line start takes its
                 // reflections in a loop (with large bodies every group does)
                 bool straight = false;
@@ -1012,55 +1060,23 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                 if (straight) {
                     if constexpr (!ROLL_J) {
 #pragma unroll
-                        for (int j = 0; j < 4; j++) reflection(g0 + j, PkNo{}, Fv[2 * j], Fv[2 * j + 1]);
+                        for (int j = 0; j < 4; j++) reflection(g0 + j, PkNo{}, Fv.v[2 * j], Fv.v[2 * j + 1]);
                     }
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 8; q++) Fv[q] = R(0);
+                    for (int q = 0; q < 8; q++) Fv.v[q] = R(0);
 #pragma unroll 1
                     for (int j = 0; j < ng; j++) {
                         R a, b;
                         reflection(g0 + j, PkYes{}, a, b);
 #pragma unroll
                         for (int q = 0; q < 4; q++)
-                            if (q == j) { Fv[2 * q] = a; Fv[2 * q + 1] = b; }
+                            if (q == j) { Fv.v[2 * q] = a; Fv.v[2 * q + 1] = b; }
                     }
                 }
-                const int o4 = width >> 1, o3 = width >> 2, o2 = width >> 3;
-                const bool b4 = lane & o4, b3 = lane & o3, b2 = lane & o2;
-                if constexpr (CEN) {
-                    // four real values over the part's lanes: halves, quarters of them, then their sums
-                    R v2[2];
-#pragma unroll
-                    for (int q = 0; q < 2; q++) {
-                        const R keep = b4 ? Fv[2 * q + 4] : Fv[2 * q], send = b4 ? Fv[2 * q] : Fv[2 * q + 4];
-                        v2[q] = keep + shfl_xor<R>(send, o4);
-                    }
-                    R v1 = (b3 ? v2[1] : v2[0]) + shfl_xor<R>(b3 ? v2[0] : v2[1], o3);
-                    for (int o = o2; o > 0; o >>= 1) v1 += shfl_xor<R>(v1, o);
-                    const int idx = (b4 ? 2 : 0) + (b3 ? 1 : 0);
-                    if ((lane & (o3 - 1)) == 0 && idx < ng) sF[wrow * ht + g0 + idx] = R2{v1, R(0)};
-                    continue;
-                }
-                // eight values over the part's lanes: halves, quarters, eighths of them, then their sums
-                R v4[4], v2[2];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const R keep = b4 ? Fv[q + 4] : Fv[q], send = b4 ? Fv[q] : Fv[q + 4];
-                    v4[q] = keep + shfl_xor<R>(send, o4);
-                }
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const R keep = b3 ? v4[q + 2] : v4[q], send = b3 ? v4[q] : v4[q + 2];
-                    v2[q] = keep + shfl_xor<R>(send, o3);
-                }
-                R v1 = (b2 ? v2[1] : v2[0]) + shfl_xor<R>(b2 ? v2[0] : v2[1], o2);
-                for (int o = o2 >> 1; o > 0; o >>= 1) v1 += shfl_xor<R>(v1, o);
-                const int idx = (b4 ? 4 : 0) + (b3 ? 2 : 0) + (b2 ? 1 : 0);
-                if ((lane & (o2 - 1)) == 0 && (idx >> 1) < ng) {
-                    R *dst = reinterpret_cast<R *>(&sF[wrow * ht + g0 + (idx >> 1)]);
-                    dst[idx & 1] = v1;
-                }
+                // (whole warps in a copy of their own, with constant lane distances)
+                if (width == 32) reduce(Fv, PkInt<32>{}, g0, ng);
+                else reduce(Fv, PkInt<0>{}, g0, ng);
             }
         } else {
             for (int i = seg0 + lane % width; i < seg0 + seg; i += width) sF[wrow * ht + i] = R2{R(0), R(0)};
