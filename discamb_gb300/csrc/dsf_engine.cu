@@ -256,6 +256,7 @@ struct dsf_structure {
     // resident tables per precision (0: FP32, 1: FP64), built when a call first needs them
     bool pk_ok[3] = {false, false, false};  // pk_kernel's records: two atoms per thread, one (FP32), FP64 (pk_kind)
     bool rs_ok[2] = {false, false}, tr_ok[2] = {false, false}, trm_ok[2] = {false, false};
+    int fp32_called = 0;  // what the last FP32 call read: 1 the radial table, 2 the kappa derivatives too
     int n_tiles_plain = 0;   // tiles [0, n_tiles_plain) hold atoms without anisotropic ADPs
     int max_types_plain = 1, max_types_aniso = 1;
     std::vector<uint8_t> active_host;
@@ -2053,9 +2054,12 @@ int dsf_structure_update_types(dsf_structure *s, const double *plm, const double
     int rc;
     if ((rc = upload_types(s))) return rc;
     if (plm && (rc = compute_global_plm(s))) return rc;
-    // the radial tables are stale: a call builds the ones of its precision (and not the other's)
+    // the radial tables are stale: a call builds the ones it reads.  The FP32 ones are built here where FP32 calls
+    // have been made (a captured one is replayed without a new call); a structure that only FP64 calls have used
+    // does without them (37 us of a cycle of 64 atoms and 16,001 reflections)
     for (int p = 0; p < 2; p++) s->tr_ok[p] = s->trm_ok[p] = false;
     refresh_dev(s);
+    if (s->fp32_called && (rc = ensure_tables(s, false, s->fp32_called == 2))) return rc;
     DSF_CUDA(cudaStreamSynchronize(e->setup));
     return DSF_OK;
 }
@@ -2140,6 +2144,7 @@ static int call_check(dsf_structure *s, int precision, int flags, const double *
         return fail(e, DSF_ERR_ARGUMENT, "dtdf and f are required");
     if (precision != DSF_FP64 && precision != DSF_FP32_BULK) return fail(e, DSF_ERR_ARGUMENT, "unknown precision");
     const bool mp = (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC;
+    if (precision != DSF_FP64) s->fp32_called = mp ? 2 : 1;
     return ensure_tables(s, precision == DSF_FP64, mp);
 }
 

@@ -163,3 +163,37 @@ def test_populations_changed_between_calls(engine):
               KEYS + ("d_plm", "d_kappa_p"), 1e-6)
         check(calc.calculate(st.dtdf, precision=api.DSF_FP32_BULK, adp_layout="padded"), ref, 1e-5, tol_f=1e-6)
         check(calc.calculate(st.dtdf, adp_layout="padded"), ref, 1e-10)
+
+
+def test_populations_changed_under_a_captured_call(engine):
+    """A captured FP32 call replayed after update_types reads the new radial tables (kappa moves
+    them all), also where no other call came between."""
+    import torch
+
+    st = shared_types("P21", 40, 8, 50, seed=6)
+    calc = api.HcCalculator(engine, st)
+    n, stream = st.n_atoms, torch.cuda.Stream()
+    dev = lambda k: torch.zeros(k, dtype=torch.float64, device="cuda")
+    out = {"f": dev(2 * st.n_hkl), "d_xyz": dev(3 * n), "d_adp": dev(6 * n), "d_occ": dev(n)}
+    g = torch.from_numpy(np.ascontiguousarray(st.dtdf).view(np.float64).ravel().copy()).cuda()
+
+    def call():
+        calc.calculate_device(g.data_ptr(), {k: v.data_ptr() for k, v in out.items()},
+                              precision=api.DSF_FP32_BULK, stream=stream.cuda_stream)
+
+    torch.cuda.synchronize()
+    call()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    kappa = np.array([1.04 * t.kappa for t in st.types])
+    for t, k in zip(st.types, kappa):
+        t.kappa = k
+    calc.update_types(kappa=kappa)
+    graph.replay()
+    torch.cuda.synchronize()
+    ref = padded(O.compute(st), st)
+    got = {k: v.cpu().numpy() for k, v in out.items()}
+    got["f"] = got["f"].view(np.complex128)
+    check({k: v.reshape(np.shape(ref[k])) for k, v in got.items()}, ref, 1e-5, tol_f=1e-6)
