@@ -402,13 +402,18 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
     if constexpr (!F64) sp += 32 * kTileAtoms;
     int *sTypes = reinterpret_cast<int *>(sp);
 
-    // Small tiles: the block's threads in `split` parts of TH / split atom slots (at least eight lanes), each part
-    // taking its own stretch of every sub-tile, so a tile of few atoms still uses every warp, every FP64 sub-unit and
-    // most lanes (an FP64 instruction costs the same however many lanes are in use)
+    // Small tiles: the block's threads in `split` parts of TH / split atom slots, each part taking its own stretch of
+    // every sub-tile, so a tile of few atoms still uses every warp and every FP64 sub-unit.  FP64: parts of eight lanes
+    // and more, of any stretch (an FP64 instruction costs the same however many lanes are in use: 32 atoms, P2_1/c,
+    // host call 172 -> 157 us).  FP32: whole warps and stretches of four reflections (the straight code's group);
+    // smaller ones start every stretch at an exact phase and add eight parts' derivatives by atomics (20 atoms, P-1,
+    // one call after another on a stream: 32 us, with parts of eight lanes 40; the constant width also takes 5,000
+    // isotropic atoms of P2_1 2_1 2_1 from 1.54 to 1.49 ms)
+    constexpr int MIN_SLOTS = F64 ? 8 : 32, MIN_SEG = F64 ? 1 : 4;
     int slots = TH;
-    while (slots > 8 && slots / 2 * NA >= n_at && ht * slots / 2 >= TH) slots >>= 1;
+    while (slots > MIN_SLOTS && slots / 2 * NA >= n_at && ht * slots / 2 >= MIN_SEG * TH) slots >>= 1;
     const int split = TH / slots, part_id = tid / slots, slot = tid - part_id * slots;
-    const int width = min(slots, 32), wrow = slot / 32;  // lanes of a part inside a warp, the warp's row of sF
+    const int width = F64 ? min(slots, 32) : 32, wrow = slot / 32;  // lanes of a part inside a warp, the warp's row of sF
     const int seg = ht / split, seg0 = part_id * seg;  // this thread's reflections of a sub-tile: [seg0, seg0 + seg)
 
     for (int i = tid; i < nT; i += TH) sTypes[i] = L.T.types[tile * kMaxTileTypes + i];
@@ -1046,7 +1051,7 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
         if (warp_any) {
 #pragma unroll 1
             for (int g0 = seg0; g0 < seg0 + seg; g0 += 4) {
-                const int ng = min(4, seg);
+                const int ng = F64 ? min(4, seg) : 4;
                 PkEight<R> Fv;
                 // a group inside its lines runs as one straight stretch of code; one with a line start takes its
                 // reflections in a loop (with large bodies every group does)
@@ -1075,8 +1080,12 @@ __device__ __forceinline__ void pk_body(const DevStructure &S, const CallBuffers
                     }
                 }
                 // (whole warps in a copy of their own, with constant lane distances)
-                if (width == 32) reduce(Fv, PkInt<32>{}, g0, ng);
-                else reduce(Fv, PkInt<0>{}, g0, ng);
+                if constexpr (!F64) {
+                    reduce(Fv, PkInt<32>{}, g0, ng);
+                } else {
+                    if (width == 32) reduce(Fv, PkInt<32>{}, g0, ng);
+                    else reduce(Fv, PkInt<0>{}, g0, ng);
+                }
             }
         } else {
             for (int i = seg0 + lane % width; i < seg0 + seg; i += width) sF[wrow * ht + i] = R2{R(0), R(0)};
