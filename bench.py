@@ -65,7 +65,7 @@ WORKLOADS = {
                     desc="config0: HC multipoles l<=4, 32 atoms (12 C, 12 H, 4 N, 4 O), P21/c, all hkl with "
                          "sin(theta)/lambda<=0.8, aniso U (H iso), dF/d(xyz,U,occ); the small-molecule case"),
     "config1": dict(seed=1, multipoles=False, flops=94, fp64_steps=3, fp64_warmup=1, cpu_frac=0.25,
-                    traffic_key="sf_grad_kernel3<float,HC,0,ISO,4,CS4,PAT_D2>@config1",
+                    traffic_key="pk_kernel<F2,HC,ISO,4,CS4,222>@config1",
                     desc="config1: HC multipoles l<=4, 5000 atoms (150 types), P212121, 54704 hkl d>=1.5A, iso B, "
                          "dF/d(xyz,B,occ)"),
     "config4": dict(seed=4, desc="config4: 256 crystals, P21/c, tabulated complex64 form factors per (atom, h'), "
