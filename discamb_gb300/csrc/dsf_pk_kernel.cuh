@@ -13,7 +13,7 @@
 //     without a branch.  Against sf_grad_body (the same box): 5,000 isotropic atoms, P2_1 2_1 2_1, 54,704
 //     reflections 1.70 -> 1.48 ms (189 warp instructions per two atoms and reflection instead of 2 x 167; the FMA
 //     pipe 60% busy, two warps per scheduler); structure factors of 8,000 atoms, 100,003 reflections 3.97 -> 3.29 ms;
-//     50,000 atoms, P4_3 2_1 2, multipole adjoint (V = float) 369 -> 308 ms; independent atoms, P2_1/c, 2,000 atoms,
+//     50,000 atoms, P4_3 2_1 2, multipole adjoint (V = float) 369 -> 300 ms; independent atoms, P2_1/c, 2,000 atoms,
 //     50,021 reflections 0.46 -> 0.26 ms (one form factor for all operations: the transform of the phases alone, and
 //     of an inversion pair only its real or imaginary half).
 //   FP64: the FP64 pipe (about 1.6 lanes per clock and SM, 1/75 of FP32), so only the number of FP64 instructions
@@ -21,7 +21,7 @@
 //     shared-memory tables plus a short polynomial (exp_tab, sincos_tab), phases are exact 64-bit fixed point, and
 //     every signed sum over a coset is a Walsh-Hadamard transform.  Against the earlier form (sf_grad_body in FP64,
 //     66-90 FP64 instructions per atom, operation and reflection, now 28-65): P2_1, 2,501 isotropic atoms, 30,011
-//     reflections 25.4 -> 10.5 ms; P4_3 2_1 2, 1,200 atoms, 20,011 reflections, multipole adjoint 34.7 -> 22.9 ms;
+//     reflections 25.4 -> 10.5 ms; P4_3 2_1 2, 1,200 atoms, 20,011 reflections, multipole adjoint 34.7 -> 23.5 ms;
 //     P2_1/c tabulated, 150 atoms, 20,021 reflections 1.58 -> 0.71 ms.  A block of four warps keeps its SM's FP64 pipe
 //     busy, so registers and occupancy do not matter here.
 // CEN: centrosymmetric structures whose inversion (at the origin) the engine takes have real adjoint weights and real
