@@ -1208,6 +1208,15 @@ int build_tiles(dsf_structure *s, bool by_type)
 
 void refresh_dev(dsf_structure *s);
 
+// While a thread builds tables its capture mode is relaxed: a call under stream capture may be the first that reads
+// them, and they are built at once on the set-up stream, outside the capture (in the default mode the allocations and
+// the wait for that stream invalidate the capture)
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // resident per-(type, reflection) radial tables; mp = the multipole-adjoint table
 // builds the tables a call of one precision needs: reflection-operation records,
 // radial terms, and (with the multipole adjoint) their kappa derivatives
@@ -1219,7 +1228,9 @@ int ensure_tables(dsf_structure *s, bool fp64, bool mp)
     const size_t esz = fp64 ? sizeof(double) : sizeof(float);
     const size_t row = 8 * (size_t)s->n_hkl_pad * std::max(1, s->n_types);
     const int pk = pk_kind(s, fp64, mp);
-    const bool built = (pk >= 0 ? !s->pk_ok[pk] : !s->rs_ok[p]) || !s->tr_ok[p] || (mp && !s->trm_ok[p]);
+    const bool build = (pk >= 0 ? !s->pk_ok[pk] : !s->rs_ok[p]) || !s->tr_ok[p] || (mp && !s->trm_ok[p]);
+    if (!build) return DSF_OK;
+    RelaxedCapture relaxed;
     if (pk >= 0 && !s->pk_ok[pk]) {
         const bool hc = s->model == MODEL_HC;
         const int nc = s->n_sym / s->pk.cs;
@@ -1246,7 +1257,7 @@ int ensure_tables(dsf_structure *s, bool fp64, bool mp)
         if (need_trm) s->trm_ok[p] = true;
     }
     // the calls that read the tables may run on another stream
-    if (built) DSF_CUDA(cudaStreamSynchronize(e->setup));
+    DSF_CUDA(cudaStreamSynchronize(e->setup));
     return DSF_OK;
 }
 

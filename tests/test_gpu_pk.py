@@ -165,6 +165,61 @@ def test_populations_changed_between_calls(engine):
         check(calc.calculate(st.dtdf, adp_layout="padded"), ref, 1e-10)
 
 
+def device_call(calc, st, multipoles):
+    """A call on device buffers as a function of its settings, its stream and its output buffers."""
+    import torch
+
+    n, stream = st.n_atoms, torch.cuda.Stream()
+    dev = lambda k: torch.zeros(k, dtype=torch.float64, device="cuda")
+    out = {"f": dev(2 * st.n_hkl), "d_xyz": dev(3 * n), "d_adp": dev(6 * n), "d_occ": dev(n)}
+    if multipoles:
+        out.update(d_pval=dev(n), d_plm=dev(25 * n), d_kappa=dev(n), d_kappa_prime=dev(n))
+    g = torch.from_numpy(np.ascontiguousarray(st.dtdf).view(np.float64).ravel().copy()).cuda()
+    torch.cuda.synchronize()
+
+    def call(precision, multipoles=multipoles):
+        calc.calculate_device(g.data_ptr(), {k: v.data_ptr() for k, v in out.items()}, precision=precision,
+                              multipoles=multipoles, stream=stream.cuda_stream)
+
+    return call, stream, out
+
+
+def check_device(out, st, precision):
+    """Output buffers of a device call against the oracle."""
+    got = {k: v.cpu().numpy() for k, v in out.items()}
+    got["f"] = got["f"].view(np.complex128)
+    if "d_kappa_prime" in got:
+        got["d_kappa_p"] = got.pop("d_kappa_prime")
+    ref = padded(O.compute(st, multipoles="d_pval" in got), st)
+    tol, tol_f = (1e-10, 1e-10) if precision == api.DSF_FP64 else (1e-5, 1e-6)
+    check({k: v.reshape(np.shape(ref[k])) for k, v in got.items()}, ref, tol, [k for k in got if k != "f"], tol_f)
+
+
+def scale_kappa(calc, st, factor):
+    kappa = np.array([factor * t.kappa for t in st.types])
+    for t, k in zip(st.types, kappa):
+        t.kappa = k
+    calc.update_types(kappa=kappa)
+
+
+@pytest.mark.parametrize("precision", [api.DSF_FP32_BULK, api.DSF_FP64])
+@pytest.mark.parametrize("multipoles", [False, True])
+def test_first_call_under_capture(engine, precision, multipoles):
+    """The first call after update_types is a captured one: it builds the tables that it reads."""
+    import torch
+
+    st = shared_types("P21", 40, 8, 50, seed=6)
+    calc = api.HcCalculator(engine, st)
+    call, stream, out = device_call(calc, st, multipoles)
+    scale_kappa(calc, st, 1.04)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call(precision)
+    graph.replay()
+    torch.cuda.synchronize()
+    check_device(out, st, precision)
+
+
 def test_populations_changed_under_a_captured_call(engine):
     """A captured FP32 call replayed after update_types reads the new radial tables (kappa moves
     them all), also where no other call came between."""
