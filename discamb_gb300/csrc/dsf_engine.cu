@@ -257,6 +257,7 @@ struct dsf_structure {
     bool pk_ok[3] = {false, false, false};  // pk_kernel's records: two atoms per thread, one (FP32), FP64 (pk_kind)
     bool rs_ok[2] = {false, false}, tr_ok[2] = {false, false}, trm_ok[2] = {false, false};
     int fp32_called = 0;  // what the last FP32 call read: 1 the radial table, 2 the kappa derivatives too
+    int captured[2] = {0, 0};  // the same of all calls made under stream capture, per precision
     int n_tiles_plain = 0;   // tiles [0, n_tiles_plain) hold atoms without anisotropic ADPs
     int max_types_plain = 1, max_types_aniso = 1;
     std::vector<uint8_t> active_host;
@@ -1261,6 +1262,15 @@ int ensure_tables(dsf_structure *s, bool fp64, bool mp)
     return DSF_OK;
 }
 
+// the tables that captured calls read, after a change of the types: their replays check nothing
+int refresh_captured(dsf_structure *s)
+{
+    int rc = DSF_OK;
+    for (int p = 0; p < 2 && !rc; p++)
+        if (s->captured[p]) rc = ensure_tables(s, p == 1, s->captured[p] == 2);
+    return rc;
+}
+
 // per-type constants of the kernels in both precisions (prefactors folded)
 template <typename R>
 TypeRadialT<R> type_constants(const TypeHost &h)
@@ -2065,12 +2075,12 @@ int dsf_structure_update_types(dsf_structure *s, const double *plm, const double
     int rc;
     if ((rc = upload_types(s))) return rc;
     if (plm && (rc = compute_global_plm(s))) return rc;
-    // the radial tables are stale: a call builds the ones it reads.  The FP32 ones are built here where FP32 calls
-    // have been made (a captured one is replayed without a new call); a structure that only FP64 calls have used
-    // does without them (37 us of a cycle of 64 atoms and 16,001 reflections)
+    // the radial tables are stale: a call builds the ones it reads.  The FP32 ones of the last FP32 call are built here;
+    // a structure that only FP64 calls have used does without them (37 us of a cycle of 64 atoms and 16,001 reflections)
     for (int p = 0; p < 2; p++) s->tr_ok[p] = s->trm_ok[p] = false;
     refresh_dev(s);
     if (s->fp32_called && (rc = ensure_tables(s, false, s->fp32_called == 2))) return rc;
+    if ((rc = refresh_captured(s))) return rc;
     DSF_CUDA(cudaStreamSynchronize(e->setup));
     return DSF_OK;
 }
@@ -2093,7 +2103,7 @@ int dsf_structure_set_electron(dsf_structure *s, int on, const int *wfn_z, const
     refresh_dev(s);
     for (int p = 0; p < 2; p++) s->tr_ok[p] = s->trm_ok[p] = false;
     if ((rc = ensure_tables(s, false, false))) return rc;
-    return DSF_OK;
+    return refresh_captured(s);
 }
 
 int dsf_structure_set_lcs(dsf_structure *s, const double *lcs)
@@ -2146,7 +2156,8 @@ double dsf_last_kernel_ms(dsf_structure *s)
 // one call, in phases: checks, adjoint weights + zeroed accumulators, the SF
 // kernel launches (one per ADP kind), the F and derivative epilogues
 // ---------------------------------------------------------------------------
-static int call_check(dsf_structure *s, int precision, int flags, const double *dtdf_device, const dsf_outputs *out)
+static int call_check(dsf_structure *s, int precision, int flags, const double *dtdf_device, const dsf_outputs *out,
+                      cudaStream_t st)
 {
     dsf_engine *e = s->eng;
     if (!s->have_hkl) return fail(e, DSF_ERR_STATE, "no reflections set");
@@ -2155,7 +2166,14 @@ static int call_check(dsf_structure *s, int precision, int flags, const double *
         return fail(e, DSF_ERR_ARGUMENT, "dtdf and f are required");
     if (precision != DSF_FP64 && precision != DSF_FP32_BULK) return fail(e, DSF_ERR_ARGUMENT, "unknown precision");
     const bool mp = (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC;
-    if (precision != DSF_FP64) s->fp32_called = mp ? 2 : 1;
+    const int reads = mp ? 2 : 1;
+    if (precision != DSF_FP64) s->fp32_called = reads;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture == cudaStreamCaptureStatusActive) {
+        int &c = s->captured[precision == DSF_FP64];
+        c = std::max(c, reads);
+    }
     return ensure_tables(s, precision == DSF_FP64, mp);
 }
 
@@ -2441,10 +2459,10 @@ int dsf_calculate_device(dsf_structure *s, int precision, int flags, const doubl
 {
     if (!s) return DSF_ERR_ARGUMENT;
     dsf_engine *e = s->eng;
-    int rc = call_check(s, precision, flags, dtdf_device, out);
-    if (rc) return rc;
     cudaSetDevice(e->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
+    int rc = call_check(s, precision, flags, dtdf_device, out, st);
+    if (rc) return rc;
     if (s->n_hkl == 0) return empty_call(s, flags, out, st);
     const bool fp64 = precision == DSF_FP64;
     const bool mp = (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC;
@@ -2640,16 +2658,16 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
     if (!structures || n < 1 || !dtdf_device || !out_device) return DSF_ERR_ARGUMENT;
     dsf_engine *e = structures[0] ? structures[0]->eng : nullptr;
     if (!e) return DSF_ERR_ARGUMENT;
+    cudaSetDevice(e->device);
+    cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
     int n_empty = 0;
     for (int i = 0; i < n; i++) {
         if (!structures[i] || structures[i]->eng != e)
             return fail(e, DSF_ERR_ARGUMENT, "batch structures must belong to one engine");
-        int rc = call_check(structures[i], precision, flags, dtdf_device[i], &out_device[i]);
+        int rc = call_check(structures[i], precision, flags, dtdf_device[i], &out_device[i], st);
         if (rc) return rc;
         n_empty += structures[i]->n_hkl == 0;
     }
-    cudaSetDevice(e->device);
-    cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
     if (n_empty) {  // structures with an empty reflection set: zero derivatives; the rest as a batch
         std::vector<dsf_structure *> sv;
         std::vector<const double *> dv;

@@ -252,3 +252,33 @@ def test_populations_changed_under_a_captured_call(engine):
     got = {k: v.cpu().numpy() for k, v in out.items()}
     got["f"] = got["f"].view(np.complex128)
     check({k: v.reshape(np.shape(ref[k])) for k, v in got.items()}, ref, 1e-5, tol_f=1e-6)
+
+
+@pytest.mark.parametrize("precision", [api.DSF_FP32_BULK, api.DSF_FP64])
+@pytest.mark.parametrize("entry", ["single", "batch"])
+def test_every_captured_call_follows_the_types(engine, precision, entry):
+    """A captured call with the multipole adjoint reads the new tables after update_types, radial terms and kappa
+    derivatives alike, also where the last call before asked for less."""
+    import torch
+
+    st = shared_types("P21", 40, 8, 50, seed=6)
+    calc = api.HcCalculator(engine, st)
+    call, stream, out = device_call(calc, st, True)
+    if entry == "batch":
+        g = torch.from_numpy(np.ascontiguousarray(st.dtdf).view(np.float64).ravel().copy()).cuda()
+        torch.cuda.synchronize()
+
+        def call(precision, multipoles=True):
+            engine.calculate_batch_device([calc], [g.data_ptr()], [{k: v.data_ptr() for k, v in out.items()}],
+                                          precision=precision, multipoles=multipoles, stream=stream.cuda_stream)
+    call(precision)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call(precision)
+    call(precision, False)
+    stream.synchronize()
+    scale_kappa(calc, st, 1.04)
+    graph.replay()
+    torch.cuda.synchronize()
+    check_device(out, st, precision)
