@@ -19,7 +19,7 @@ PEAK_LIB = os.path.join(HERE, "libdsf_peak_probe.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["dsf_kernels.cu", "dsf_k3_f32_hc.cu", "dsf_k3_f32_hc_mp.cu", "dsf_k3_f32_other.cu", "dsf_k3b_f32.cu", "dsf_k3_f64.cu", "dsf_prep_kernels.cu", "dsf_engine.cu", "dsf_noalloc.cu", "dsf_tsc.cu", "dsf_k3f_hc.cu", "dsf_k3f_other.cu",
            "dsf_pk_f64_hc.cu", "dsf_pk_f64_hc_mp.cu", "dsf_pk_f64_hc_f.cu", "dsf_pk_f64_iam.cu", "dsf_pk_f64_table.cu",
-           "dsf_pk_f32_hc.cu", "dsf_pk_f32_hc_f.cu", "dsf_pk_f32_hc_mp.cu", "dsf_pk_f32_hc_batch.cu", "dsf_pk_f32_iam.cu",
+           "dsf_pk_f32_hc.cu", "dsf_pk_f32_hc_f.cu", "dsf_pk_f32_hc_mp.cu", "dsf_pk_f32_hc_batch.cu", "dsf_pk_f32_iam.cu", "dsf_pk_f32_iam_f.cu",
            "dsf_pk_f32_iam_batch.cu", "dsf_pk_f32_hc1.cu", "dsf_pk_f32_hc1_f.cu", "dsf_pk_f32_hc1_batch.cu"]
 
 

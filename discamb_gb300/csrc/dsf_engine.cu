@@ -2415,7 +2415,8 @@ static int launch_pk_structure(dsf_structure *s, int kind, bool mp, bool grad, i
     const int want = std::max(1, (s->n_hkl + n_chunks0 - 1) / n_chunks0);
     const bool hc = s->model == MODEL_HC;
     mp = mp && hc;
-    int rc = pk_setup(s, kind, mp, grad || !hc, want, ht_cap, C, L, A.smem);
+    // (FP64 has no kernels without the derivatives for the generic models)
+    int rc = pk_setup(s, kind, mp, grad || (!hc && kind == 2), want, ht_cap, C, L, A.smem);
     if (rc) return rc;
     L.hkl_chunk = (want + L.ht - 1) / L.ht * L.ht;
     A.S = &s->dev;
@@ -2427,7 +2428,7 @@ static int launch_pk_structure(dsf_structure *s, int kind, bool mp, bool grad, i
     A.st = st;
     A.split_kinds = (long long)A.n_tiles * A.n_chunks >= 16ll * e->n_sm;
     cudaError_t ce;
-    if (s->model == MODEL_IAM) ce = kind == 2 ? launch_pk_f64_iam(A) : launch_pk_f32_iam(A);
+    if (s->model == MODEL_IAM) ce = kind == 2 ? launch_pk_f64_iam(A) : grad ? launch_pk_f32_iam(A) : launch_pk_f32_iam_f(A);
     else if (s->model == MODEL_TABLE) ce = launch_pk_f64_table(A);
     else if (mp) ce = kind == 2 ? launch_pk_f64_hc_mp(A) : launch_pk_f32_hc_mp(A);
     else if (grad) ce = kind == 2 ? launch_pk_f64_hc(A) : kind == 1 ? launch_pk_f32_hc1(A) : launch_pk_f32_hc(A);

@@ -145,6 +145,7 @@ cudaError_t launch_pk_f64_table(const PkArgs &A);
 cudaError_t launch_pk_f32_hc(const PkArgs &A);
 cudaError_t launch_pk_f32_hc_f(const PkArgs &A);
 cudaError_t launch_pk_f32_iam(const PkArgs &A);
+cudaError_t launch_pk_f32_iam_f(const PkArgs &A);
 cudaError_t launch_pk_f32_hc_mp(const PkArgs &A);
 cudaError_t launch_pk_f32_hc_batch(const PkArgs &A);
 cudaError_t launch_pk_f32_hc1(const PkArgs &A);

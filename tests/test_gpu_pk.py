@@ -282,3 +282,22 @@ def test_every_captured_call_follows_the_types(engine, precision, entry):
     graph.replay()
     torch.cuda.synchronize()
     check_device(out, st, precision)
+
+
+def random_iam(st, seed, terms=4):
+    rng = np.random.default_rng(seed)
+    nt = int(st.atom_type.max()) + 1
+    return dict(ngauss=np.full(nt, terms, np.int32), a=rng.uniform(.5, 3, (nt, 5)), b=rng.uniform(.5, 30, (nt, 5)),
+                c=rng.uniform(0, .5, nt))
+
+
+@pytest.mark.parametrize("sg", ["P1", "P-1", "P21", "P21/c", "C2/c", "P212121", "Pbca", "P43212", "P3"])
+@pytest.mark.parametrize("n_atoms", [5, 37, 130])
+def test_independent_atoms_structure_factors_only(engine, sg, n_atoms):
+    """derivatives=(): the forward-only kernels of the FP32 independent-atom model, and the FP64 call."""
+    st = W.small_case(sg, n_atoms=n_atoms, stol_max=0.35, seed=78, n_types=6)
+    iam = random_iam(st, 3)
+    calc = api.IamCalculator(engine, st, iam)
+    ref = O.compute(st, model="iam", iam=iam)["f"]
+    for precision, tol in ((api.DSF_FP32_BULK, 1e-6), (api.DSF_FP64, 1e-10)):
+        assert rel_f(calc.calculate(st.dtdf, precision=precision, derivatives=())["f"], ref) < tol
