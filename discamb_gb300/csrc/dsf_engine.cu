@@ -2424,7 +2424,7 @@ static int launch_pk_structure(dsf_structure *s, int kind, bool mp, bool grad, i
     A.L = &L;
     A.form = s->pk;
     A.n_tiles = n_tiles;
-    A.n_chunks = (s->n_hkl + L.hkl_chunk - 1) / L.hkl_chunk;
+    A.n_chunks = L.n_chunks = (s->n_hkl + L.hkl_chunk - 1) / L.hkl_chunk;
     A.st = st;
     A.split_kinds = (long long)A.n_tiles * A.n_chunks >= 16ll * e->n_sm;
     cudaError_t ce;

@@ -340,6 +340,7 @@ struct PkNo {
 
 struct PkLaunch {
     int hkl_chunk, ht, n_hkl_pad;
+    int n_chunks;          // reflection chunks of a tile (pk_kernel)
     PkTiles T;
     const void *pk;        // reflection records
     const void *tr, *trm;  // R [n_types][n_hkl_pad][8]
@@ -1167,7 +1168,8 @@ __host__ __device__ constexpr int pk_min_blocks()
     return sizeof(V) == 4 && !MP ? 4 : 1;
 }
 
-// one structure: block (reflection chunk, tile), so that blocks that run together share a tile's code and types.  KIND
+// one structure: block tile * n_chunks + reflection chunk, so that blocks that run together share a tile's code and types
+// (one grid dimension: a structure has any number of tiles, the others hold 65,535).  KIND
 // 2: both ADP kinds in one launch (FP64, and FP32 grids of a few blocks per SM, where a second launch costs more than
 // it saves); 0, 1: one launch per kind (two kinds' code at once overflow the instruction caches)
 template <typename V, int MODEL, bool MP, int NSC, int CS, bool GRAD, bool INV, int PAT, bool CEN, int KIND>
@@ -1176,7 +1178,7 @@ pk_kernel(const __grid_constant__ DevStructure S, const __grid_constant__ CallBu
           const __grid_constant__ PkLaunch L)
 {
     pk_tile<V, MODEL, MP, NSC, CS, GRAD, INV, PAT, CEN, KIND, KIND == 2>(
-        S, C, L, blockIdx.y + (KIND == 1 ? L.T.n_plain : 0), blockIdx.x);
+        S, C, L, blockIdx.x / L.n_chunks + (KIND == 1 ? L.T.n_plain : 0), blockIdx.x % L.n_chunks);
 }
 
 // many structures of one kernel form in one launch (kernel-parameter space holds up to kBatchItems): the block's item

@@ -85,7 +85,7 @@ cudaError_t launch_pk_tiles(K k, int threads, int n_tiles, const PkArgs &A)
     if (n_tiles <= 0) return cudaSuccess;
     cudaError_t e = dynamic_smem(k, A.smem);
     if (e != cudaSuccess) return e;
-    k<<<dim3(A.n_chunks, n_tiles), threads, A.smem, A.st>>>(*A.S, *A.C, *A.L);
+    k<<<A.n_chunks * n_tiles, threads, A.smem, A.st>>>(*A.S, *A.C, *A.L);
     return cudaGetLastError();
 }
 

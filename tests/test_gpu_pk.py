@@ -301,3 +301,34 @@ def test_independent_atoms_structure_factors_only(engine, sg, n_atoms):
     ref = O.compute(st, model="iam", iam=iam)["f"]
     for precision, tol in ((api.DSF_FP32_BULK, 1e-6), (api.DSF_FP64, 1e-10)):
         assert rel_f(calc.calculate(st.dtdf, precision=precision, derivatives=())["f"], ref) < tol
+
+
+def test_more_tiles_than_a_grid_dimension_holds(engine):
+    """65,537 tiles: copies of a 128-atom cell with occupancies of their own.  F is the small cell's times the sum of
+    the factors, an atom's derivatives the small cell's (by position and ADP times its factor)."""
+    copies = 65537
+    st = W.small_case("P1", n_atoms=128, stol_max=0.35, seed=31, n_types=5)
+    st.adp = np.random.default_rng(2).uniform(0.02, 0.05, (128, 6)) * np.array([1, 1, 1, .2, .2, .2])
+    st = cut(st, 3)
+    iam = random_iam(st, 3)
+    ref = O.compute(st, model="iam", iam=iam)
+    factor = np.random.default_rng(4).uniform(0.5, 1.5, copies)
+    big = W.small_case("P1", n_atoms=128, stol_max=0.35, seed=31, n_types=5)
+    big.hkl, big.dtdf = st.hkl, st.dtdf
+    big.xyz, big.adp = np.tile(st.xyz, (copies, 1)), np.tile(st.adp, (copies, 1))
+    big.occupancy = np.outer(factor, st.occupancy).ravel()
+    for k in ("multiplicity", "atom_wfn", "atom_type"):
+        setattr(big, k, np.tile(getattr(st, k), copies))
+    if st.anomalous is not None:
+        big.anomalous = np.tile(st.anomalous, copies)
+    calc = api.IamCalculator(engine, big, iam)
+    want = {"d_xyz": np.multiply.outer(factor, ref["d_xyz"]).reshape(-1, 3),
+            "d_adp": np.multiply.outer(factor, np.array(ref["d_adp"])).reshape(-1, 6), "d_occ": np.tile(ref["d_occ"], copies)}
+    for precision, tol in ((api.DSF_FP64, 1e-10), (api.DSF_FP32_BULK, 1e-5)):
+        got = calc.calculate(big.dtdf, precision=precision, adp_layout="padded")
+        assert rel_f(got["f"], ref["f"] * factor.sum()) < min(tol, 1e-6)
+        for k, v in want.items():
+            assert rel_norm(got[k], v) < tol, k
+            # no tile left out: the largest difference of any atom
+            assert np.abs(got[k] - v).max() < 10 * tol * np.abs(v).max(), k
+    calc.close()
