@@ -96,4 +96,14 @@ struct CallBuffers {
     double *g_acc;         // [n_atoms][kNch]
 };
 
+// The opt-in that a launch with more than 48 KB of dynamic shared memory needs: always the device's largest size, so
+// that threads that launch one kernel with different sizes cannot lower it for one another between this and the launch
+constexpr int kMaxDynamicSmem = 227 * 1024;
+template <typename K>
+inline cudaError_t allow_dynamic_smem(K kernel, size_t bytes)
+{
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+}
+
 }  // namespace dsf

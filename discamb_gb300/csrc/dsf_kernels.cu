@@ -483,7 +483,7 @@ template <typename R, bool MP>
 cudaError_t launch_sf_grad_t(const DevStructure &S, const CallBuffers &C, int hkl_chunk, int ht, cudaStream_t st)
 {
     const size_t smem = sf_grad_smem<R>(ht, S.n_sym);
-    cudaError_t e = cudaFuncSetAttribute(sf_grad_kernel<R, MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(sf_grad_kernel<R, MP>, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(S.n_tiles, (S.n_hkl + hkl_chunk - 1) / hkl_chunk);
     sf_grad_kernel<R, MP><<<grid, kTileAtoms, smem, st>>>(S, C, hkl_chunk, ht);

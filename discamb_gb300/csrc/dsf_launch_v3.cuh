@@ -29,7 +29,7 @@ struct K3Args {
 template <typename K, typename... Args>
 cudaError_t launch_with(K k, dim3 grid, size_t smem, cudaStream_t st, const Args &...args)
 {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<grid, kTileAtoms, smem, st>>>(args...);
     return cudaGetLastError();

@@ -71,19 +71,11 @@ inline bool pk_generic_form(const PkForm &f, F &&go)
     return false;
 }
 
-// the opt-in that a launch needs above 48 KB of dynamic shared memory
-template <typename K>
-cudaError_t dynamic_smem(K k, size_t bytes)
-{
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 template <typename K>
 cudaError_t launch_pk_tiles(K k, int threads, int n_tiles, const PkArgs &A)
 {
     if (n_tiles <= 0) return cudaSuccess;
-    cudaError_t e = dynamic_smem(k, A.smem);
+    cudaError_t e = allow_dynamic_smem(k, A.smem);
     if (e != cudaSuccess) return e;
     k<<<A.n_chunks * n_tiles, threads, A.smem, A.st>>>(*A.S, *A.C, *A.L);
     return cudaGetLastError();
@@ -109,7 +101,7 @@ template <typename V, int MODEL, typename C>
 cudaError_t launch_pk_batch(const PkArgs &A)
 {
     auto k = pk_batch_kernel<V, MODEL, C::N, C::CS, C::INV, C::PAT, C::CEN>;
-    cudaError_t e = dynamic_smem(k, A.smem);
+    cudaError_t e = allow_dynamic_smem(k, A.smem);
     if (e != cudaSuccess) return e;
     k<<<A.blocks, pk_threads<V>(), A.smem, A.st>>>(*A.B);
     return cudaGetLastError();

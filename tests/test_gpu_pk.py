@@ -332,3 +332,40 @@ def test_more_tiles_than_a_grid_dimension_holds(engine):
             # no tile left out: the largest difference of any atom
             assert np.abs(got[k] - v).max() < 10 * tol * np.abs(v).max(), k
     calc.close()
+
+
+def test_two_threads_with_different_shared_memory(engine):
+    """Two host threads launch one kernel with 5 and with 32 types per tile (other shared-memory sizes) at once: FP64
+    batches, which launch per structure."""
+    import threading
+
+    import torch
+
+    failed, jobs = [], []
+    for n_types in (5, 60):
+        st = shared_types("P1", 120, n_types, 16, seed=8)
+        calcs = [api.HcCalculator(engine, st) for _ in range(16)]
+        parts = [device_call(c, st, True) for c in calcs]
+        g = torch.from_numpy(np.ascontiguousarray(st.dtdf).view(np.float64).ravel().copy()).cuda()
+        jobs.append((st, calcs, [p[2] for p in parts], g, parts[0][1]))
+    torch.cuda.synchronize()
+
+    def many(st, calcs, outs, g, stream):
+        try:
+            for _ in range(200):
+                engine.calculate_batch_device(calcs, [g.data_ptr()] * len(calcs),
+                                              [{k: v.data_ptr() for k, v in o.items()} for o in outs],
+                                              precision=api.DSF_FP64, multipoles=True, stream=stream.cuda_stream)
+        except api.DsfError as exc:
+            failed.append(exc)
+
+    threads = [threading.Thread(target=many, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed
+    for st, _, outs, _, _ in jobs:
+        for out in outs:
+            check_device(out, st, api.DSF_FP64)
