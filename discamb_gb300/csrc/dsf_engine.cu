@@ -2156,8 +2156,15 @@ double dsf_last_kernel_ms(dsf_structure *s)
 // one call, in phases: checks, adjoint weights + zeroed accumulators, the SF
 // kernel launches (one per ADP kind), the F and derivative epilogues
 // ---------------------------------------------------------------------------
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) cudaGetLastError();
+    return c == cudaStreamCaptureStatusActive;
+}
+
 static int call_check(dsf_structure *s, int precision, int flags, const double *dtdf_device, const dsf_outputs *out,
-                      cudaStream_t st)
+                      bool captured)
 {
     dsf_engine *e = s->eng;
     if (!s->have_hkl) return fail(e, DSF_ERR_STATE, "no reflections set");
@@ -2168,9 +2175,7 @@ static int call_check(dsf_structure *s, int precision, int flags, const double *
     const bool mp = (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC;
     const int reads = mp ? 2 : 1;
     if (precision != DSF_FP64) s->fp32_called = reads;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
-    if (capture == cudaStreamCaptureStatusActive) {
+    if (captured) {
         int &c = s->captured[precision == DSF_FP64];
         c = std::max(c, reads);
     }
@@ -2462,7 +2467,7 @@ int dsf_calculate_device(dsf_structure *s, int precision, int flags, const doubl
     dsf_engine *e = s->eng;
     cudaSetDevice(e->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
-    int rc = call_check(s, precision, flags, dtdf_device, out, st);
+    int rc = call_check(s, precision, flags, dtdf_device, out, capturing(st));
     if (rc) return rc;
     if (s->n_hkl == 0) return empty_call(s, flags, out, st);
     const bool fp64 = precision == DSF_FP64;
@@ -2661,11 +2666,12 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
     if (!e) return DSF_ERR_ARGUMENT;
     cudaSetDevice(e->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
+    const bool captured = capturing(st);
     int n_empty = 0;
     for (int i = 0; i < n; i++) {
         if (!structures[i] || structures[i]->eng != e)
             return fail(e, DSF_ERR_ARGUMENT, "batch structures must belong to one engine");
-        int rc = call_check(structures[i], precision, flags, dtdf_device[i], &out_device[i], st);
+        int rc = call_check(structures[i], precision, flags, dtdf_device[i], &out_device[i], captured);
         if (rc) return rc;
         n_empty += structures[i]->n_hkl == 0;
     }
