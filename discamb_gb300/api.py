@@ -123,6 +123,7 @@ def library():
         L.dsf_tsc_load.argtypes = [C.c_char_p, _P(C.c_int), _P(C.c_int), _P(C.c_int), _P(C.c_double), C.c_int]
         L.dsf_form_factors.argtypes = [C.c_void_p, _P(C.c_int), _P(C.c_int), _P(C.c_double)]
         L.dsf_debug_stall_next_call.argtypes = [C.c_void_p]
+        L.dsf_debug_kernel_kind.argtypes = [C.c_void_p, C.c_int, C.c_int]
         L.dsf_structure_set_anomalous.argtypes = [C.c_void_p, _P(C.c_double)]
         L.dsf_submit.argtypes = [C.c_void_p, C.c_int, C.c_int, _P(C.c_double), _P(C.c_double), _P(C.c_double),
                                  _P(C.c_double), _P(C.c_int), _P(_Out), _P(C.c_void_p)]
@@ -419,6 +420,11 @@ class _Calculator:
         next call's kernel waits run out and the call raises DsfError
         (DSF_ERR_TIMEOUT) after about 4 s; the engine stays usable."""
         self.engine.check(self.lib.dsf_debug_stall_next_call(self.h), "debug_stall_next_call")
+
+    def debug_kernel_kind(self, precision=DSF_FP64, derivatives=("xyz", "adp", "occ"), multipoles=False):
+        """Test hook (dsf_debug_kernel_kind): -1 the general kernel, 0 two atoms
+        per thread (FP32), 1 one (FP32), 2 FP64."""
+        return self.lib.dsf_debug_kernel_kind(self.h, int(precision), _flags(derivatives, multipoles))
 
     def form_factors(self, hkl, include=None):
         """The single-h calculateFormFactors of the reference

@@ -735,9 +735,15 @@ bool fractional_signs(dsf_structure *s, int cs)
     return true;
 }
 
-// The operations' form for pk_kernel: cosets of four or two consecutive operations whose relative maps flip axes as
-// a compiled sign group does (HC: the Cartesian maps of the harmonics too), the second half of the operations as
-// inversion images (generic models), or no cosets (cs = 1)
+// whether pk_kernel is compiled for a form of the model's operations
+bool pk_compiled(int model, const PkForm &f)
+{
+    return model == MODEL_HC ? pk_hc_form(f, [](auto) {}) : pk_generic_form(f, [](auto) {});
+}
+
+// The operations' form for pk_kernel, the first of these that is compiled: cosets of four or two consecutive operations
+// whose relative maps flip axes as a sign group does (HC: the Cartesian maps of the harmonics too), with the second half
+// of the operations as inversion images where they are (generic models), or no cosets (cs = 1); cs = 0: none is
 PkForm pk_form_of(const dsf_structure *s)
 {
     const int n = s->n_sym;
@@ -768,38 +774,29 @@ PkForm pk_form_of(const dsf_structure *s)
         }
         return true;
     };
-    PkForm f;
-    f.n_sym = n;
-    f.inv = !hc && s->inv_pairs != 0;
-    f.cen = hc && s->centro_mode == 1;
+    auto form = [&](int cs, int pat) {
+        PkForm f;
+        f.n_sym = n;
+        f.cs = cs;
+        f.pat = pat;
+        f.inv = !hc && cs > 1 && s->inv_pairs != 0;
+        f.cen = hc && n == cs && s->centro_mode == 1;
+        return f;
+    };
     for (const int pat : {kPatD2, kPatC2hB})
-        if (cosets(4, pat & 7, pat >> 3)) {
-            f.cs = 4;
-            f.pat = pat;
-            f.cen = f.cen && n == 4;
-            return f;
-        }
+        if (cosets(4, pat & 7, pat >> 3) && pk_compiled(s->model, form(4, pat))) return form(4, pat);
     for (const int a : {kPat2Y, kPat2Z, kPatInv})
-        if (cosets(2, a, 0)) {
-            f.cs = 2;
-            f.pat = a;
-            f.cen = f.cen && n == 2;
-            return f;
-        }
-    f.cs = 1;
-    f.inv = false;
-    f.cen = f.cen && n == 1;
-    return f;
+        if (cosets(2, a, 0) && pk_compiled(s->model, form(2, a))) return form(2, a);
+    return pk_compiled(s->model, form(1, 0)) ? form(1, 0) : PkForm{};
 }
 
 // the record kind (and thread value) pk_kernel takes a call in: 0 FP32 with two atoms per thread, 1 FP32 with one
-// (multipole adjoint; a type per atom), 2 FP64; -1: the call's form or model has no pk_kernel (FP32 tables stream through registers in
-// sf_grad_body; sign groups and operation counts that are not compiled)
+// (multipole adjoint; a type per atom), 2 FP64; -1: the call's form or model has no pk_kernel (FP32 tables stream
+// through registers in sf_grad_body; sign groups and operation counts that are not compiled)
 int pk_kind(const dsf_structure *s, bool fp64, bool mp)
 {
     if (s->model == MODEL_TABLE && !fp64) return -1;
-    const bool form = s->model == MODEL_HC ? pk_hc_form(s->pk, [](auto) {}) : pk_generic_form(s->pk, [](auto) {});
-    if (!form) return -1;
+    if (s->pk.cs == 0) return -1;
     if (fp64) return 2;
     return s->model == MODEL_HC && (mp || !s->pk_pairs) ? 1 : 0;
 }
@@ -3237,6 +3234,11 @@ int dsf_debug_stall_next_call(dsf_structure *s)
     if (!s) return DSF_ERR_ARGUMENT;
     s->debug_stall = 1;
     return DSF_OK;
+}
+
+int dsf_debug_kernel_kind(const dsf_structure *s, int precision, int flags)
+{
+    return s ? pk_kind(s, precision == DSF_FP64, (flags & DSF_D_MULTIPOLE) && s->model == MODEL_HC) : -1;
 }
 
 int dsf_form_factors(dsf_structure *s, const int *hkl, const int *include, double *ff)

@@ -255,6 +255,9 @@ int dsf_form_factors(dsf_structure *s, const int *hkl, const int *include, doubl
  * and a host-buffer call returns DSF_ERR_TIMEOUT; the engine stays usable.  No reference counterpart (the reference
  * GPU code exit()s on errors, src/GPU/cuda/globals.h:22). */
 int dsf_debug_stall_next_call(dsf_structure *s);
+/* test hook: the kernel that a call with these settings takes: -1 the general one, 0 two atoms per thread (FP32), 1 one
+ * atom per thread (FP32), 2 FP64 with one atom per thread */
+int dsf_debug_kernel_kind(const dsf_structure *s, int precision, int derivative_flags);
 /* asynchronous dsf_calculate_atoms for serving (xyz/adp/occupancy may be NULL: the resident atoms): the inputs are
  * staged before the call returns (the caller may reuse its input buffers at once), the kernels and the readback
  * are queued on the engine's stream, and *ticket identifies the call.  The output buffers are written by dsf_poll.

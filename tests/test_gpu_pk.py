@@ -369,3 +369,48 @@ def test_two_threads_with_different_shared_memory(engine):
     for st, _, outs, _, _ in jobs:
         for out in outs:
             check_device(out, st, api.DSF_FP64)
+
+
+# operation lists in the usual order, beside those of crystal.SPACE_GROUPS
+LISTS = {
+    "P4/m": "x,y,z;-x,-y,z;-y,x,z;y,-x,z;-x,-y,-z;x,y,-z;y,-x,-z;-y,x,-z",
+    "P422, 222 first": "x,y,z;-x,-y,z;x,-y,-z;-x,y,-z;-y,x,z;y,-x,z;y,x,-z;-y,-x,-z",
+}
+HC, BOTH = ("hc",), ("hc", "iam", "table")
+
+
+@pytest.mark.parametrize("sg,models", [("P1", BOTH), ("P-1", BOTH), ("P21", BOTH), ("P21/c", BOTH), ("C2/c", BOTH),
+                                       ("P212121", BOTH), ("Pbca", BOTH), ("P41", HC), ("P43212", BOTH),
+                                       ("P422, 222 first", BOTH), ("P4/m", BOTH), ("P3", ()), ("Fdd2", ())])
+def test_which_kernel_a_listed_group_takes(engine, sg, models):
+    """Every group whose operations have a compiled form takes pk_kernel (its records' kind), the others the general
+    kernel, and FP32 tables always that."""
+    from discamb_gb300.crystal import SpaceGroup
+    st = W.small_case("P43212" if sg in LISTS else sg, n_atoms=12, stol_max=0.3, seed=3, n_types=5)
+    if sg in LISTS:
+        st.sg = SpaceGroup(sg, LISTS[sg].split(";"))
+    ops = len(api.all_ops_mod_centering(st.sg)[0])
+    calcs = {"hc": api.HcCalculator(engine, st), "iam": api.IamCalculator(engine, st, random_iam(st, 3)),
+             "table": api.TabulatedCalculator(engine, st, np.ones((st.n_hkl, ops, 12), complex))}
+    for model, calc in calcs.items():
+        kinds = [calc.debug_kernel_kind(api.DSF_FP32_BULK), calc.debug_kernel_kind(api.DSF_FP32_BULK, multipoles=True),
+                 calc.debug_kernel_kind(api.DSF_FP64)]
+        want = [-1, -1, -1] if model not in models else {"hc": [0, 1, 2], "iam": [0, 0, 2], "table": [-1, -1, 2]}[model]
+        assert kinds == want, model
+
+
+@pytest.mark.parametrize("sg", list(LISTS))
+def test_eight_operations_without_compiled_cosets(engine, sg):
+    """Generic models with eight operations in no compiled coset form, against the oracle."""
+    from discamb_gb300.crystal import SpaceGroup
+    st = W.small_case("P43212", n_atoms=37, stol_max=0.35, seed=77)
+    st.sg = SpaceGroup(sg, LISTS[sg].split(";"))
+    iam = random_iam(st, 3)
+    rng = np.random.default_rng(3)
+    table = rng.normal(size=(st.n_hkl, 8, 37)) + 1j * rng.normal(size=(st.n_hkl, 8, 37))
+    for calc, ref in ((api.IamCalculator(engine, st, iam), O.compute(st, model="iam", iam=iam)),
+                      (api.TabulatedCalculator(engine, st, table), O.compute(st, model="table", table=table))):
+        ref = padded(ref, st)
+        check(calc.calculate(st.dtdf, adp_layout="padded"), ref, 1e-10)
+        check(calc.calculate(st.dtdf, precision=api.DSF_FP32_BULK, adp_layout="padded"), ref, 1e-5, tol_f=1e-6)
+        check(engine.calculate_batch([calc], [st.dtdf])[0], ref, 1e-5, tol_f=1e-6)
