@@ -2310,13 +2310,14 @@ static int chunk_count(const dsf_engine *e, int ntk, int n_hkl, int blocks_per_s
 static int log2_bucket(double x) { return x > 1 ? (int)std::lround(2.0 * std::log2(x)) : 0; }
 
 // the shape a structure's call depends on: model, precision, multipole adjoint, derivative pass, operation
-// count, coset form, atoms and reflections in half-octaves, the device's SM count
+// count, coset form, the kernel (pk_kind; -1: sf_grad_body) and its form, atoms and reflections in half-octaves,
+// the device's SM count
 static std::string tune_key(const dsf_structure *s, bool fp64, bool mp, bool grad)
 {
     char k[160];
-    std::snprintf(k, sizeof k, "m%d-p%d-mp%d-g%d-ns%d-cs%d-iv%d-a%d-h%d-sm%d", s->model, fp64 ? 64 : 32, mp ? 1 : 0,
-                  grad ? 1 : 0, s->n_sym, s->coset_size, s->inv_pairs, log2_bucket(s->n_atoms),
-                  log2_bucket(s->n_hkl), s->eng->n_sm);
+    std::snprintf(k, sizeof k, "m%d-p%d-mp%d-g%d-ns%d-cs%d-iv%d-k%d.%d.%d.%d-a%d-h%d-sm%d", s->model, fp64 ? 64 : 32,
+                  mp ? 1 : 0, grad ? 1 : 0, s->n_sym, s->coset_size, s->inv_pairs, pk_kind(s, fp64, mp), s->pk.cs,
+                  s->pk.pat, s->pk.cen ? 1 : 0, log2_bucket(s->n_atoms), log2_bucket(s->n_hkl), s->eng->n_sm);
     return k;
 }
 
@@ -2633,9 +2634,8 @@ int dsf_tuning_save(dsf_engine *e, const char *path)
     return DSF_OK;
 }
 
-// adds the shapes of a file written by dsf_tuning_save (the third number, once a register-capped form, is read and
-// not used; keys name the device's SM count, so shapes tuned on
-// another kind of device are never matched)
+// adds the shapes of a file written by dsf_tuning_save (the third number, once a register-capped form, is read and not
+// used; keys name the kernel and the device's SM count, so shapes tuned for another kernel or device are never matched)
 int dsf_tuning_load(dsf_engine *e, const char *path)
 {
     if (!e || !path) return DSF_ERR_ARGUMENT;

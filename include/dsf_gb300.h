@@ -287,8 +287,8 @@ int dsf_calculate_batch_atoms(dsf_structure *const *structures, int n, int preci
  * the structure's call (these precision and derivative flags) over a few tile shapes -- reflection chunks aiming
  * at 24, 48, 75 or 150 blocks per SM, the longest shared-memory sub-tile or at most 8 reflections -- on a zero
  * dT/dF in scratch buffers it allocates and frees, and keeps the fastest for every later call of structures with the
- * same shape key (model, precision, multipole adjoint, derivative pass, operation count, coset form, atoms and
- * reflections in half-octaves, SM count).  Results do not depend on the shape beyond the order of the
+ * same shape key (model, precision, multipole adjoint, derivative pass, operation count, coset form, kernel,
+ * atoms and reflections in half-octaves, SM count).  Results do not depend on the shape beyond the order of the
  * cross-block sums.  Synchronous.  dsf_tuning_lookup: the shape the next call would take (ht 0: the longest
  * sub-tile; occupancy: always 0; *tuned 0: the rule, 75 blocks per SM).  dsf_tuning_save / dsf_tuning_load: the engine's tuned shapes to and from a text file. */
 int dsf_autotune(dsf_structure *s, int precision, int derivative_flags, int *blocks_per_sm, int *ht,

@@ -71,3 +71,34 @@ def test_register_capped_form_keeps_the_results(engine):
     o = O.compute(st, multipoles=True)
     assert rel_f(r1["f"], o["f"]) < tf
     calc.close()
+
+
+def test_a_shape_is_for_one_kernel(engine):
+    # the same atoms, reflections and operations with shared types (two atoms per thread) and with a type per atom
+    # (one): a shape tuned for the one is not the other's, nor is one saved for a kernel that the key does not name
+    prec = api.DSF_FP32_BULK
+    shared, own = (api.HcCalculator(engine, W.small_case("P212121", n_atoms=230, stol_max=0.55, seed=37, n_types=k))
+                   for k in (6, None))
+    assert (shared.debug_kernel_kind(prec), own.debug_kernel_kind(prec)) == (0, 1)
+    assert not shared.tile_shape(prec)["tuned"]
+    own.autotune(prec)
+    assert own.tile_shape(prec)["tuned"] and not shared.tile_shape(prec)["tuned"]
+    own.close()
+    shared.close()
+
+
+def test_a_file_of_shapes_without_the_kernel_matches_nothing(engine, tmp_path):
+    import re
+    prec = api.DSF_FP32_BULK
+    calc = api.HcCalculator(engine, W.small_case("P212121", n_atoms=90, stol_max=0.5, seed=41))
+    calc.autotune(prec)
+    path = tmp_path / "tuning.txt"
+    engine.save_tuning(str(path))
+    path.write_text(re.sub(r"-k[-\d.]+-a", "-a", path.read_text()))
+    other = api.Engine(0)
+    c2 = api.HcCalculator(other, calc.st)
+    other.load_tuning(str(path))
+    assert not c2.tile_shape(prec)["tuned"]
+    c2.close()
+    other.close()
+    calc.close()
