@@ -72,15 +72,24 @@ class _Entry:
 
 
 def estimate_device_bytes(n_atoms, n_hkl, n_sym, n_types=1, multipoles=False):
-    """Device bytes of one structure for FP32 calls: reflection-operation
-    records, radial tables per (type, reflection), per-reflection and
-    per-atom buffers."""
+    """Device bytes of one structure for FP32 calls, an upper bound over the
+    kernels: reflection records, radial tables per (type, reflection),
+    per-reflection, per-atom and per-type buffers."""
     n_pad = (n_hkl + 15) // 16 * 16
-    rs = n_pad * n_sym * 144
+    # records of a reflection: the general kernel's, 144 bytes per operation, or pk_kernel's, 32 per operation and 272
+    # per coset of operations (144 more for the multipole adjoint, which has records of its own); the symmetry forms
+    # of four and eight operations have up to two cosets
+    cosets = 1 if n_sym <= 2 else 2
+    pairs = 32 * n_sym + 272 * cosets + (32 * n_sym + 144 * cosets if multipoles else 0)
+    rec = n_pad * max(144 * n_sym, pairs)
     tr = n_types * n_pad * 8 * 4 * (2 if multipoles else 1)
-    per_h = n_pad * (16 * 4 + 8 * 4 + 8 * 6)
-    per_atom = n_atoms * (8 * 40 + 8 * 25 * 2 + 165 * 8 + 8 * 30)
-    return rs + tr + per_h + per_atom
+    # h, |h|^2 in both precisions, multiplier, inversion phase, dT/dF, adjoint weights, F accumulator, F, order, flags
+    per_h = n_pad * (16 + 12 + 8 + 16 + 16 + 24 + 16 + 16 + 8)
+    # derivative accumulator, populations (both precisions), rotation blocks, inputs twice, outputs, frame, line steps;
+    # coordinates, ADPs, weights, dispersion and indices; the tiles' slots (32 types close a tile of 128)
+    per_atom = n_atoms * (8 * 40 + 12 * 25 + 8 * 165 + 2 * 80 + 8 * 38 + 8 * 9 + 24 * n_sym + 208 + 96)
+    per_type = n_types * (8 * 25 + 512)
+    return rec + tr + per_h + per_atom + per_type + 65536
 
 
 def batch_executor(engine, precision=api.DSF_FP32_BULK, derivatives=("xyz", "adp", "occ")):

@@ -163,3 +163,19 @@ def test_request_in_a_mixed_batch_equals_the_call_alone(engine, precision, tf, t
         for q in ("d_xyz", "d_adp", "d_occ"):
             assert rel_norm(r[q], a[q]) < tg, (k, q, rel_norm(r[q], a[q]))
     srv.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sg", ["P1", "P-1", "P21", "P21/c", "P212121", "C2/c", "P41", "P43212", "P3", "Pbca"])
+@pytest.mark.parametrize("n_types", [20, None])
+@pytest.mark.parametrize("multipoles", [False, True])
+def test_admission_estimate_holds_what_a_structure_takes(engine, sg, n_types, multipoles):
+    """No structure takes more than its estimate after an FP32 host-buffer call, nor less than a third of it."""
+    from discamb_gb300 import api, workloads as W
+    st = W.small_case(sg, n_atoms=150, stol_max=0.6, seed=17, n_types=n_types)
+    calc = api.HcCalculator(engine, st)
+    calc.calculate(st.dtdf, precision=api.DSF_FP32_BULK, multipoles=multipoles,
+                   atoms=(st.xyz, st.adp, st.occupancy))
+    est = serve.estimate_device_bytes(st.n_atoms, st.n_hkl, len(st.sg.subset_rot), len(st.types), multipoles)
+    assert est / 3 < calc.device_bytes() <= est
+    calc.close()
