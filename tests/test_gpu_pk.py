@@ -414,3 +414,56 @@ def test_eight_operations_without_compiled_cosets(engine, sg):
         check(calc.calculate(st.dtdf, adp_layout="padded"), ref, 1e-10)
         check(calc.calculate(st.dtdf, precision=api.DSF_FP32_BULK, adp_layout="padded"), ref, 1e-5, tol_f=1e-6)
         check(engine.calculate_batch([calc], [st.dtdf])[0], ref, 1e-5, tol_f=1e-6)
+
+
+def many_blocks(sg, n_types):
+    """8,000 atoms of both ADP kinds and 10,240 reflections in whole lattice lines: 63 and more tiles in chunks of 256
+    reflections are over 16 blocks per SM, where FP32 calls take one launch per ADP kind."""
+    cell = (64.0, 64.0, 72.0, 90.0, 90.0, 90.0)
+    laue = {"P1": 2, "P-1": 2, "P21": 4, "P21/c": 4, "P41": 8, "P212121": 8, "Pbca": 8, "P43212": 16}[sg]
+    rng = np.random.default_rng(60)
+    # reflections to s: 4/3 pi (2 s)^3 V, one in `laue` of them unique, and a third more
+    stol = (1.35 * 10240 * laue / (32 * np.pi / 3 * 64 * 64 * 72)) ** (1 / 3)
+    st = W.build_structure(cell=cell, sg_symbol=sg, elements=W.protein_elements(8000, rng), rng=rng, n_types=n_types,
+                           stol_max=stol)
+    order = np.lexsort(st.hkl.T[::-1])[:10240]
+    st.hkl, st.dtdf = np.ascontiguousarray(st.hkl[order]), st.dtdf[order]
+    assert st.n_hkl == 10240 and len(set(map(len, st.adp))) == 2
+    return st
+
+
+def against_fp64(calc, st, **kw):
+    a = calc.calculate(st.dtdf, precision=api.DSF_FP64, adp_layout="padded", **kw)
+    b = calc.calculate(st.dtdf, precision=api.DSF_FP32_BULK, adp_layout="padded", **kw)
+    assert rel_f(b["f"], a["f"]) < 1e-6
+    for k in a:
+        if k != "f" and kw.get("derivatives") != ():
+            assert rel_norm(b[k], a[k]) < 1e-5, k
+
+
+@pytest.mark.parametrize("sg", ["P1", "P-1", "P21", "P21/c", "P41", "P212121", "Pbca", "P43212"])
+def test_fp32_one_launch_per_adp_kind(engine, sg):
+    """Calls large enough for a launch per ADP kind, with straight groups of reflections, against the FP64 call."""
+    st = many_blocks(sg, 60)
+    calc = api.HcCalculator(engine, st)
+    assert calc.debug_kernel_kind(api.DSF_FP32_BULK) == 0
+    against_fp64(calc, st)
+    against_fp64(calc, st, multipoles=True)
+    against_fp64(calc, st, derivatives=())
+    calc.close()
+    calc = api.IamCalculator(engine, st, random_iam(st, 3))
+    against_fp64(calc, st)
+    against_fp64(calc, st, derivatives=())
+    calc.close()
+
+
+@pytest.mark.parametrize("sg", ["P1", "P-1", "P212121", "P43212"])
+def test_fp32_one_launch_per_adp_kind_a_type_per_atom(engine, sg):
+    """The same with types of one or two atoms: one atom per thread."""
+    st = many_blocks(sg, 6000)
+    calc = api.HcCalculator(engine, st)
+    assert calc.debug_kernel_kind(api.DSF_FP32_BULK) == 1
+    against_fp64(calc, st)
+    against_fp64(calc, st, multipoles=True)
+    against_fp64(calc, st, derivatives=())
+    calc.close()
