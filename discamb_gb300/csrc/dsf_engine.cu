@@ -798,6 +798,13 @@ int pk_kind(const dsf_structure *s, bool fp64, bool mp)
     if (s->model == MODEL_TABLE && !fp64) return -1;
     if (s->pk.cs == 0) return -1;
     if (fp64) return 2;
+    // small isotropic structures with eight operations in no coset form fill the SMs better with one atom per thread
+    // (P4_3 2_1 2, independent atoms, sf_grad_body | pk_kernel: 200 atoms, 6,001 reflections 42 | 44 us, F only 37 | 42;
+    // 400 atoms, 12,001 reflections 79 | 81; 800 atoms, 24,001 reflections 269 | 219; anisotropic ones 66 | 58, 118 | 110,
+    // 348 | 342)
+    if (s->model == MODEL_IAM && s->pk.cs == 1 && s->n_sym == 8 && s->n_tiles_plain == s->n_tiles &&
+        (double)s->n_atoms * s->n_hkl < 8e6)
+        return -1;
     return s->model == MODEL_HC && (mp || !s->pk_pairs) ? 1 : 0;
 }
 
@@ -2903,7 +2910,10 @@ int dsf_calculate_batch_device(dsf_structure *const *structures, int n, int prec
             PKB.n = m;
             double pairs = 0;
             for (int k = 0; k < m; k++) pairs += (double)pk_map(g.items[b0 + k], g.kind).n_tiles * g.items[b0 + k]->n_hkl;
-            const int want = (int)std::max(64.0, pairs / (std::max(1, e->n_sm) * 24.0));
+            // (eight operations in no coset form take longer per reflection: chunks down to 32 reflections; ten
+            // independent-atom crystals of up to 150 atoms, P4_3 2_1 2: 135 -> 120 us, sf_grad_batch3 130)
+            const double least = g.model != MODEL_HC && g.form.cs == 1 && g.form.n_sym == 8 ? 32.0 : 64.0;
+            const int want = (int)std::max(least, pairs / (std::max(1, e->n_sm) * 24.0));
             int blocks = 0;
             PkArgs A;
             for (int k = 0; k < m; k++) {

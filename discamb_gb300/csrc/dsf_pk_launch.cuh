@@ -32,7 +32,7 @@ constexpr int kPat2Y = 5, kPat2Z = 3, kPatInv = 7;  // cs = 2: a two-fold axis a
 //   HC (operations without the inversion): P1 and P-1; P2_1, P2_1/c, C2/c; P4_1; 222; 422
 //   other models (all operations modulo centring): 1; 2; -1; 222; 2/m; mmm; any eight.  Eight in no compiled coset
 //   form (P4_3 2_1 2 as listed, 4/m) against sf_grad_body, independent atoms: FP32, 2,000 atoms, 50,021 reflections
-//   1,422 -> 1,089 us (isotropic 839 -> 769); FP64, 500 atoms, 10,001 reflections 7,762 -> 2,798 us; tabulated in FP64,
+//   1,448 -> 1,130 us (isotropic 867 -> 770); FP64, 500 atoms, 10,001 reflections 7,762 -> 2,798 us; tabulated in FP64,
 //   150 atoms, 20,021 reflections 5,484 -> 2,790 us
 template <int N_, int CS_, int PAT_, bool INV_ = false, bool CEN_ = false>
 struct PkC {

@@ -467,3 +467,21 @@ def test_fp32_one_launch_per_adp_kind_a_type_per_atom(engine, sg):
     against_fp64(calc, st, multipoles=True)
     against_fp64(calc, st, derivatives=())
     calc.close()
+
+
+@pytest.mark.parametrize("n_hkl,kind", [(1000, -1), (10240, 0)])
+def test_isotropic_independent_atoms_with_eight_operations(engine, n_hkl, kind):
+    """Isotropic structures with eight operations in no coset form take the general kernel when they are small; both
+    sides of the rule against the FP64 call."""
+    st = many_blocks("P43212", 60)
+    st.adp = [a[:1] for a in st.adp]
+    st = st.subset(np.arange(900))
+    st.hkl, st.dtdf = st.hkl[:n_hkl], st.dtdf[:n_hkl]
+    iam = random_iam(st, 3)
+    calc = api.IamCalculator(engine, st, iam)
+    assert calc.debug_kernel_kind(api.DSF_FP32_BULK) == kind
+    against_fp64(calc, st)
+    against_fp64(calc, st, derivatives=())
+    a = calc.calculate(st.dtdf, adp_layout="padded")
+    check(engine.calculate_batch([calc], [st.dtdf])[0], a, 1e-5, tol_f=1e-6)
+    calc.close()
