@@ -76,7 +76,7 @@ WORKLOADS = {
                                  "hkl log-uniform 1k-300k, P1/P-1/P21/P21c/P212121/C2c, HC l<=4, aniso U, "
                                  "dF/d(xyz,U,occ)"),
     "config2": dict(seed=2, multipoles=True, flops=195, fp64_steps=1, fp64_warmup=0, cpu_frac=0.002,
-                    traffic_key=None,
+                    traffic_key="pk_kernel<float,HC,MP,8,CS4,222>@config2",
                     desc="config2: HC multipoles l<=4, 50000 atoms (300 types), P43212, all hkl d>=1.2A, aniso U "
                          "(H iso), dF/d(xyz,U,occ,Pv,Plm,kappa,kappa')"),
 }
@@ -794,6 +794,8 @@ def run_gpu(args, served=None):
                      "peak_source": "FP32 FMA throughput probe measured in this run (MEASURED_PEAKS.json lists "
                                     "HBM and bf16 tensor peaks only)",
                      "flops_per_term": wl["flops"], "kernel_ms": k32,
+                     "flops_note": "the formulas' operations, term by term; the kernels execute fewer, so frac is "
+                                   "not the FMA pipe's load (55-60%, profiles/pk_kernel_fp32.md)",
                      "hbm_peak_gbs_measured": mp.get("hbm_gbs")},
         "cpu_baseline": {"value": cpu_v, "unit": "terms/s", "cores": os.cpu_count() or 1, "kind": "port",
                          "sample": f"{args.workload} atoms x first {cpu_m // 2} and {cpu_m} reflections (C time "
@@ -803,7 +805,6 @@ def run_gpu(args, served=None):
         "clocks": {"sm_mhz": clocks["sm_mhz"], "sm_max_mhz": clocks["sm_max_mhz"], "reasons": clocks["reasons"]},
         "wall_s_timed_region": wall32,
         "tile_shape": {"blocks_per_sm": shape["blocks_per_sm"], "ht": shape["ht"] or "longest",
-                       "register_cap_blocks_per_sm": shape["occupancy"] or "compiler's",
                        "source": "autotuner (dsf_autotune at set-up)" if shape["tuned"]
                        else "rule (75 blocks per SM, longest sub-tile)",
                        "tuned_ms": tuned["ms"] if tuned else None},

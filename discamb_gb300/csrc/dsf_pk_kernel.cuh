@@ -135,7 +135,7 @@ __device__ __forceinline__ double exp_tab(double x, const double *tab)
 }
 
 // sin and cos of 2 pi P 2^-64: the nearest of kSinN directions from the table, the remainder (|x| <= pi / kSinN) by
-// Taylor polynomials to x^5 and x^6 (truncation below 1e-17), and their product; 15 FP64 instructions
+// Taylor polynomials to x^5 and x^6 (truncation below 1e-17), and their product; 13 FP64 instructions
 __device__ __forceinline__ void sincos_tab(uint64_t P, const double *tab, double *sn, double *cs)
 {
     const uint32_t j = (uint32_t)((P + (1ull << 54)) >> 55) & (kSinN - 1);
