@@ -208,6 +208,7 @@ int dsf_structure_destroy(dsf_structure *s);
 int dsf_structure_set_hkl(dsf_structure *s, int n_hkl, const int *hkl);
 /* atoms in the crystal's conventions; adp [n_atoms][6] (first 1 or 6 used) */
 int dsf_structure_update_atoms(dsf_structure *s, const double *xyz, const double *adp, const double *occupancy);
+/* NULL arguments keep their values; replays of calls captured into a CUDA graph see the new types */
 int dsf_structure_update_types(dsf_structure *s, const double *type_plm, const double *type_pval,
                                const double *type_kappa, const double *type_kappa_prime);
 int dsf_structure_set_lcs(dsf_structure *s, const double *lcs);
